@@ -12,6 +12,7 @@
 
 #include "acoustic_step2.cuh"
 #include "adjoint_kernels.cuh"
+#include "resident.cuh"
 #include "small_kernels.cuh"
 #include "w2d_common.cuh"
 #include "wave2d_cuda.h"
@@ -145,8 +146,14 @@ struct w2d_engine {
     bool vel_set[2] = {false, false};
     DevBuf<float> staging;  // one plane, pitched upload area
 
-    DevBuf<int> shot;  // {src_ix, src_iz, rec_iz}
-    int h_shot[3] = {-1, -1, -1};  // host copy of the same
+    DevBuf<int> shot;  // {src_ix, src_iz, rec_iz, n_rec, rec_c0}
+    int h_shot[5] = {-1, -1, -1, 0, -1};  // host copy of the same
+    bool one_per_column = true;           // no column holds two receivers
+
+    // resident form (resident.cu): how the grid is cut into tiles that stay on
+    // chip (no plan where it does not fit), and the packets its tiles exchange
+    RsPlan rs;
+    DevBuf<uint4> rs_x;
     DevBuf<int> rec_ptr, rec_list;
     DevBuf<float> wavelet, data, rec_out;
     DevBuf<float> snaps, ckpt;
@@ -401,9 +408,9 @@ int set_shot(w2d_engine* e, int src_ix, int src_iz, const int* rec_ix, int n_rec
         (rc = e->shot.ensure(5)))
         return rc;
     int sh[5] = {src_ix, src_iz, rec_iz, n_rec, receivers_consecutive_c0(rec_ix, n_rec)};
-    e->h_shot[0] = src_ix;
-    e->h_shot[1] = src_iz;
-    e->h_shot[2] = rec_iz;
+    std::copy(sh, sh + 5, e->h_shot);
+    e->one_per_column = true;
+    for (int i = 0; i < e->nx; ++i) e->one_per_column &= ptr[i + 1] - ptr[i] <= 1;
     W2D_CUDA_TRY(cudaMemcpyAsync(e->rec_ptr.p, ptr.data(), ptr.size() * 4, cudaMemcpyHostToDevice,
                                  e->stream));
     W2D_CUDA_TRY(cudaMemcpyAsync(e->rec_list.p, list.data(), list.size() * 4,
@@ -421,6 +428,56 @@ AcStep base_step(w2d_engine* e)
     s.dt2_inj = (float)(e->dt_d * e->dt_d);
     s.err = e->err.p;
     return s;
+}
+
+// Whether the steps of a pass run in the resident form: the default launch mode, a grid
+// that fits the chip, and a source and receivers that the kernel takes.
+bool resident(const w2d_engine* e, int n_rec, bool with_source)
+{
+    return e->rs.ok() && !e->persistent && e->pdl && !e->two_step && !e->l2_hints &&
+           rs_shot_fits(e->nx, e->nz, with_source ? e->h_shot[0] : -1, e->h_shot[1], n_rec,
+                        e->h_shot[2], e->one_per_column);
+}
+
+// The shot as the resident kernel takes it, without what a pass reads and writes.
+RsShot rs_shot(w2d_engine* e)
+{
+    RsShot s{};
+    s.nx = e->nx;
+    s.nz = e->nz;
+    s.ldx = e->ldx;
+    s.gx = e->rs.gx;
+    s.gz = e->rs.gz;
+    s.maxc = e->rs.maxc;
+    s.maxr = e->rs.maxr;
+    s.inv_dx2 = e->inv_dx2;
+    s.inv_dz2 = e->inv_dz2;
+    s.fs = e->fs;
+    s.n_sponge = e->n_sponge;
+    s.lut = e->use_lut ? e->sponge_lut.p : nullptr;
+    s.src_ix = e->h_shot[0];
+    s.src_iz = e->h_shot[1];
+    s.rec_iz = e->h_shot[2];
+    s.n_rec = e->h_shot[3];
+    s.rec_c0 = e->h_shot[4];
+    s.rec_ptr = e->rec_ptr.p;
+    s.rec_list = e->rec_list.p;
+    for (int i = 0; i < 6; ++i) s.wave[i] = e->wave(i);
+    s.plane = e->plane;
+    s.dt2_inj = (float)(e->dt_d * e->dt_d);
+    s.xbuf = e->rs_x.p;
+    s.err = e->err.p;
+    return s;
+}
+
+// Phase steps [s.k0, s.k1) in one launch.
+int rs_run(w2d_engine* e, const RsShot& s)
+{
+    // no packet of an earlier launch may carry one of this launch's tags
+    W2D_CUDA_TRY(cudaMemsetAsync(e->rs_x.p, 0, e->rs.xbuf_bytes(), e->stream));
+    W2D_CUDA_TRY(launch_acoustic_resident(s, nullptr, nullptr, e->rs.ctas(), e->stream));
+    e->last_launches++;
+    return W2D_OK;
 }
 
 // Forward steps [it0, it1) on the forward triple (roles by it % 3).
@@ -449,6 +506,8 @@ int run_forward_steps(w2d_engine* e, int slot, const FwdOpts& o, int it0, int it
             if (o.illum) s.illum = e->illum.p;
         }
     };
+    // (a recomputed segment samples no receivers, but they are on the device all the same)
+    const bool on_chip = resident(e, e->h_shot[3], true);
     for (int it = it0; it < it1;) {
         if (o.ckpt && o.ckpt_every > 0 && it % o.ckpt_every == 0) {
             e->chain = false;
@@ -459,6 +518,26 @@ int run_forward_steps(w2d_engine* e, int slot, const FwdOpts& o, int it0, int it
                                          cudaMemcpyDeviceToDevice, e->stream));
             W2D_CUDA_TRY(cudaMemcpyAsync(c + 2 * e->plane, e->wave((it + 2) % 3), e->plane * 4,
                                          cudaMemcpyDeviceToDevice, e->stream));
+        }
+        if (on_chip) {  // up to the next checkpoint in one launch
+            RsShot r = rs_shot(e);
+            r.nt = o.nt;
+            r.interval = o.interval;
+            r.k0 = it;
+            r.k1 = o.ckpt && o.ckpt_every > 0
+                       ? std::min(it1, (it / o.ckpt_every + 1) * o.ckpt_every)
+                       : it1;
+            r.vel[0] = e->v2dt2.p + (size_t)slot * e->plane;
+            r.snaps = o.snaps;
+            r.slot0 = o.slot0;
+            r.illum = o.illum ? e->illum.p : nullptr;
+            r.wavelet = e->cur_w;
+            r.rec_out = o.rec_out;
+            r.dt2_inj = dt2inj_f;
+            int rc;
+            if ((rc = rs_run(e, r))) return rc;
+            it = r.k1;
+            continue;
         }
         // two steps in one launch unless a checkpoint falls between them
         const bool pair = e->two_step && !e->persistent && it + 1 < it1 &&
@@ -517,6 +596,23 @@ int run_backward_steps(w2d_engine* e, int slot, int nt, int interval, int n_rec,
             }
         }
     };
+    if (resident(e, n_rec, false)) {
+        RsShot r = rs_shot(e);
+        r.src_ix = -1;
+        r.nt = nt;
+        r.interval = interval;
+        r.k0 = 2 * nt - 1 - it_hi;
+        r.k1 = 2 * nt - it_lo;
+        r.vel[1] = e->v2dt2.p + (size_t)slot * e->plane;
+        r.snaps = const_cast<float*>(snaps);
+        r.slot0 = slot0;
+        r.n_snaps = n_snaps_valid;
+        r.image = snaps ? e->image.p : nullptr;
+        r.data = e->cur_data;
+        r.img_dt = img_dt;
+        r.dt2_inj = dt2inj_f;
+        return rs_run(e, r);
+    }
     for (int it = it_hi; it >= it_lo;) {
         const int m = nt - 1 - it;
         int rc;
@@ -573,10 +669,13 @@ std::vector<uintptr_t> pass_key(const w2d_engine* e, int pass, int nt, int inter
 // from `body` (the host code that launches it), instantiate and launch the graph.  With
 // graphs off, or in a launch mode that keeps host-side state, `body` runs directly.  A
 // capture the runtime refuses turns graphs off for this engine and runs `body`.
+// Nor a pass in the resident form: it is a launch or two as it is, by shot-specific
+// arguments.
 template <typename F>
-int run_pass(w2d_engine* e, w2d_engine::PassGraph& pg, std::vector<uintptr_t> key, F&& body)
+int run_pass(w2d_engine* e, w2d_engine::PassGraph& pg, std::vector<uintptr_t> key, bool on_chip,
+             F&& body)
 {
-    if (!e->use_graphs || e->two_step || e->persistent) return body();
+    if (!e->use_graphs || e->two_step || e->persistent || on_chip) return body();
     if (pg.exec && pg.key == key) {
         W2D_CUDA_TRY(cudaGraphLaunch(pg.exec, e->stream));
         e->last_launches += pg.launches;
@@ -703,6 +802,7 @@ int w2d_engine_create(w2d_engine** out, int nx, int nz, float dx, float dz, doub
         return fail(W2D_ECUDA);
     }
     // Sponge: a Cerjan table when the array is one, else the array itself.
+    bool lut_ok = true;
     if (sponge) {
         // recover (n, alpha) candidates from the array: n is the largest frame
         // distance with a value != 1; alpha from the value at distance 1 is not
@@ -739,6 +839,7 @@ int w2d_engine_create(w2d_engine** out, int nx, int nz, float dx, float dz, doub
         if (ok) {
             e->n_sponge = n;
             lut[0] = 1.0f;
+            lut_ok = rs_lut_fits(lut.data(), n);
             if ((rc = e->sponge_lut.ensure(n + 1))) return fail(rc);
             cudaMemcpy(e->sponge_lut.p, lut.data(), (n + 1) * 4, cudaMemcpyHostToDevice);
             e->use_lut = true;
@@ -757,6 +858,10 @@ int w2d_engine_create(w2d_engine** out, int nx, int nz, float dx, float dz, doub
     cudaMemcpy(e->shot.p, sh, sizeof sh, cudaMemcpyHostToDevice);
     cudaMemset(e->rec_ptr.p, 0, (nx + 1) * 4);
     if ((rc = ensure_tensor_maps(e))) return fail(rc);
+    if (!e->use_arr && (!e->use_lut || lut_ok)) {
+        e->rs = rs_plan(nx, nz, rs_capacity());
+        if (e->rs.ok() && (rc = e->rs_x.ensure(e->rs.xbuf_bytes() / sizeof(uint4)))) return fail(rc);
+    }
     if (cudaDeviceSynchronize() != cudaSuccess) {
         set_error("engine set-up failed");
         return fail(W2D_ECUDA);
@@ -784,6 +889,7 @@ void w2d_engine_destroy(w2d_engine* e)
     e->err.release();
     e->scratch.release();
     e->tile_counter.release();
+    e->rs_x.release();
     for (auto& b : e->st_w) b.release();
     for (auto& b : e->st_d) b.release();
     if (e->t0) cudaEventDestroy(e->t0);
@@ -924,7 +1030,7 @@ int w2d_forward(w2d_engine* e, int vel_slot, const float* wavelet, int nt, int s
     };
     const int kind = (vel_slot << 2) | (snaps_out ? 1 : 0) | (n_rec > 0 ? 2 : 0);
     if ((rc = run_pass(e, e->g_model, pass_key(e, 2, nt, snapshot_interval, kind, 0, n_rec),
-                       pass)))
+                       resident(e, n_rec, true), pass)))
         return rc;
     cudaEventRecord(e->ev1, e->stream);
     if (n_rec > 0)
@@ -993,7 +1099,8 @@ int w2d_backward_correlate(w2d_engine* e, int vel_slot, const float* data, int n
                                   dt2inj);
     };
     if ((rc = run_pass(e, e->g_bcorr,
-                       pass_key(e, 3, nt, snapshot_interval, vel_slot, n_snaps, n_rec), pass)))
+                       pass_key(e, 3, nt, snapshot_interval, vel_slot, n_snaps, n_rec),
+                       resident(e, n_rec, false), pass)))
         return rc;
     cudaEventRecord(e->ev1, e->stream);
     if ((rc = download_field(e, image, e->image.p))) return rc;
@@ -1074,7 +1181,8 @@ int migrate_core(w2d_engine* e, int nt, int n_rec, int snapshot_interval, int st
         W2D_CUDA_TRY(cudaGetLastError());
         return W2D_OK;
     };
-    if ((rc = run_pass(e, e->g_fwd, pass_key(e, 0, nt, interval, mode, seg, n_rec), forward)))
+    if ((rc = run_pass(e, e->g_fwd, pass_key(e, 0, nt, interval, mode, seg, n_rec),
+                       resident(e, n_rec, true), forward)))
         return rc;
     if (image_out) W2D_CUDA_TRY(cudaEventRecord(e->fwd_done, e->stream));
 
@@ -1117,7 +1225,9 @@ int migrate_core(w2d_engine* e, int nt, int n_rec, int snapshot_interval, int st
         }
         return W2D_OK;
     };
-    if ((rc = run_pass(e, e->g_bwd, pass_key(e, 1, nt, interval, mode, seg, n_rec), backward)))
+    // (with checkpoints it recomputes forward segments: on chip as a whole or not at all)
+    if ((rc = run_pass(e, e->g_bwd, pass_key(e, 1, nt, interval, mode, seg, n_rec),
+                       resident(e, n_rec, mode != W2D_STORE_ALL), backward)))
         return rc;
     cudaEventRecord(e->ev1, e->stream);
     if (image_out) {

@@ -1,0 +1,137 @@
+// resident.cuh -- the acoustic time loop with its wavefields kept on chip (resident.cu): which
+// shots it takes, how a grid is cut into tiles, and the launch.
+#pragma once
+
+#include <algorithm>
+
+#include "w2d_common.cuh"
+
+namespace w2d {
+
+constexpr int RS_CT = 480;          // compute threads (15 warps)
+constexpr int RS_T = RS_CT + 32;    // and one halo warp: 16 warps, 128 registers a thread
+constexpr int RS_MAXR = 15;         // rows of one phase-I thread: its tensor-memory words
+constexpr int RS_SMEM = 227 * 1024; // always the whole SM: no second CTA, which could wait
+                                    // for tensor memory while its neighbours wait for it
+constexpr int RS_POLLS = 1 << 21;    // looks at a missing packet before giving up (about 1 s)
+constexpr int RS_FLIGHT = 11;       // packets a halo lane has in flight
+
+// One shot (or one pass of it) as the resident kernel runs it.  Phase step k is forward
+// step k for k < nt, else backward step 2*nt-1-k.
+struct RsShot {
+    int nx, nz, ldx, gx, gz, maxc, maxr;
+    float inv_dx2, inv_dz2;
+    int fs, n_sponge;
+    const float* lut;          // sponge by frame distance, non-increasing (null: none)
+    int src_ix, src_iz, rec_iz, n_rec, rec_c0;
+    const int* rec_ptr;        // at most one receiver per column
+    const int* rec_list;
+    int nt, interval, k0, k1;
+    float* wave[6];            // forward triple, backward triple, roles by step as elsewhere
+    const float* vel[2];       // v^2 dt^2 of the forward and the backward pass
+    float* snaps;              // forward: written when not null; backward: read when imaging
+    int slot0, n_snaps;        // first snapshot held; snapshots that exist (backward)
+    size_t plane;
+    float* illum;              // forward: accumulated when not null
+    float* image;              // backward: accumulated when not null
+    const float* wavelet;
+    const float* data;
+    float* rec_out;            // forward: sampled when not null
+    float dt2_inj, img_dt;
+    float minus_zero = -0.0f;  // an operand the compiler must not know (see mul2)
+    uint4* xbuf;               // packets: tile, slot, {left, right, top, bottom}
+    unsigned* err;
+};
+
+// ---- host: how a grid is cut -------------------------------------------------------
+struct RsPlan {
+    int gx = 0, gz = 0, maxc = 0, maxr = 0;
+    bool ok() const { return gx > 0; }
+    int ctas() const { return gx * gz; }
+    size_t packets() const { return 2 * (size_t)(2 * maxr + 8 * maxc); }  // of one tile
+    size_t xbuf_bytes() const { return packets() * ctas() * sizeof(uint4); }
+};
+
+constexpr int RS_TILE_FLOATS = 64, RS_SHOT_FLOATS = 96;  // the tile's and the shot's records
+
+// floats of shared memory of a tile of nrows x ncol units
+__host__ __device__ inline size_t rs_smem_floats(int nrows, int ncol)
+{
+    const size_t pitch = 4 * (size_t)ncol;
+    return RS_TILE_FLOATS + RS_SHOT_FLOATS + 2 * (nrows + 4) * pitch + 8 * (size_t)nrows + 4 * pitch + (nrows + 3) / 4 * 4 + 16;
+}
+
+// Phase I of a tile: columns 1..ncol-2 by rows 2..nrows-3 in segments of R rows.
+__host__ __device__ inline void rs_interior(int nrows, int ncol, int* nci, int* nseg, int* R)
+{
+    *nci = ncol - 2;
+    const int ni = nrows - 4;
+    *nseg = *R = 0;
+    if (*nci <= 0 || ni <= 0) return;
+    const int s = min(RS_CT / *nci, ni);
+    *R = (ni + s - 1) / s;
+    *nseg = (ni + *R - 1) / *R;
+}
+
+// The cut of an nx x nz grid into at most max_ctas tiles with the least estimated step
+// time: what a step costs is its slowest tile, so columns and rows are split evenly and
+// the estimate (in cycles) is that of the largest tile.  No plan when the grid does not
+// fit the SMs' shared memory.
+inline RsPlan rs_plan(int nx, int nz, int max_ctas)
+{
+    RsPlan best;
+    double best_cost = 1e30;
+    const int w4 = (nx + 3) / 4;
+    for (int gx = 1; gx <= max_ctas && (gx == 1 || w4 / gx >= 2); ++gx)
+        for (int gz = 1; gx * gz <= max_ctas && (gz == 1 || nz / gz >= 4); ++gz) {
+            const int ncol = (w4 + gx - 1) / gx, nrows = (nz + gz - 1) / gz;
+            const int ne = 2 * nrows + 4 * (ncol - 2);
+            if (ncol < 2 || nrows < 5 - (gz > 1) || ne > RS_CT) continue;
+            if (rs_smem_floats(nrows, ncol) * 4 > (size_t)RS_SMEM) continue;
+            int nci, nseg, R;
+            rs_interior(nrows, ncol, &nci, &nseg, &R);
+            if (R > RS_MAXR) continue;
+            const double warps = std::max(1.0, nci * nseg / 32.0);
+            const double inner = R ? (R + 1.5) * std::max(warps / 4 * 75.0, 150.0) : 0.0;
+            const double cost = 600.0 + ne / 128.0 * 110.0 + inner +
+                                std::max(0.0, 1200.0 - inner) + 0.5 * gx * gz;
+            if (cost < best_cost) {
+                best_cost = cost;
+                best.gx = gx;
+                best.gz = gz;
+                best.maxc = ncol;
+                best.maxr = nrows;
+            }
+        }
+    return best;
+}
+
+// The sources and receivers the kernel takes: on interior rows (and columns, for the
+// source), at most one receiver per column.  src_ix < 0: no source.
+inline bool rs_shot_fits(int nx, int nz, int src_ix, int src_iz, int n_rec, int rec_iz,
+                         bool unique_columns)
+{
+    if (src_ix >= 0 && (src_ix < 2 || src_ix >= nx - 2 || src_iz < 2 || src_iz >= nz - 2))
+        return false;
+    return n_rec == 0 || (unique_columns && rec_iz >= 2 && rec_iz < nz - 2);
+}
+
+// The sponge as a product of nothing but the larger frame distance's factor needs
+// factors that do not increase with distance: lut[max(a, b)] = min(lut[a], lut[b]).
+inline bool rs_lut_fits(const float* lut, int n)
+{
+    for (int d = 0; d <= n; ++d)
+        if (!(lut[d] <= (d ? lut[d - 1] : 1.0f)) || (d == 0 && lut[d] != 1.0f)) return false;
+    return true;
+}
+
+// Phase steps of one shot, or (many) of several, items[CTA] = {shot, tile}: one cooperative
+// launch of `ctas` CTAs.  Packets of earlier launches must be gone from xbuf.
+cudaError_t launch_acoustic_resident(const RsShot& one, const RsShot* many, const int2* items,
+                                     int ctas, cudaStream_t st);
+
+// CTAs that are resident at once on the current device (0 on error or where a
+// cooperative launch is not available).
+int rs_capacity();
+
+}  // namespace w2d

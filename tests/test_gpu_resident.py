@@ -1,0 +1,68 @@
+"""The time loop with its wavefields kept on chip (the default where a grid fits) against
+one launch per step: traces, snapshots, images and illumination bit-identical.
+
+Sizes: the smallest grid, every remainder of nx by the four-point unit, one tile, many
+tiles, tiles of the least height, the production grid; calls that keep the step kernels
+(receivers sharing a column, sources and receivers off the interior rows) are among them.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+# nz, nx, free surface, sponge, receiver row, receivers, interval, steps
+CASES = [
+    (5, 5, True, 0, 2, "all", 1, 7),
+    (8, 6, False, 2, 3, "all", 2, 9),
+    (9, 37, True, 3, 2, "all", 1, 1),
+    (33, 130, True, 6, 2, "all", 2, 41),
+    (34, 131, True, 6, 3, "third", 3, 40),
+    (35, 129, False, 6, 20, "shuffled", 2, 40),
+    (61, 260, True, 10, 58, "all", 1, 33),
+    (61, 261, True, 10, 2, "shared", 2, 33),
+    (61, 262, False, 10, 1, "all", 2, 33),
+    (150, 403, True, 40, 2, "all", 4, 120),
+    (607, 1203, False, 30, 36, "third", 2, 90),
+    (1000, 4000, True, 40, 2, "all", 2, 60),
+    (1024, 4096, True, 40, 2, "all", 2, 12),  # beyond the chip
+]
+
+
+@pytest.mark.parametrize("nz,nx,fs,n_sponge,riz,kind,interval,nt", CASES)
+def test_resident_equals_steps(nz, nx, fs, n_sponge, riz, kind, interval, nt):
+    from das_gb300.rtm_engine import TSWRTMEngine
+    from das_gb300.velocity_flood import FloodModels
+    from das_gb300.wave_solver import WaveSolver2D
+    rng = np.random.default_rng(nz * 5000 + nx)
+    v = rng.uniform(1500, 3000, (nz, nx)).astype(np.float32)
+    v2 = (v * np.float32(1.01)).astype(np.float32)
+    w = rng.standard_normal(nt).astype(np.float32)
+    rix = {"all": np.arange(nx), "third": np.arange(1, nx, 3),
+           "shuffled": rng.permutation(nx)[: nx // 2],
+           "shared": np.sort(rng.integers(0, nx, nx // 2))}[kind]
+    data = rng.standard_normal((nt, len(rix))).astype(np.float32)
+    out = []
+    for pdl in (True, False):  # the default launch mode, and the step kernels
+        s = WaveSolver2D(nx, nz, 5.0, 5.0, 5e-4, n_sponge=n_sponge, free_surface_top=fs)
+        s.set_launch("grid", pdl)
+        six, siz = max(2, nx // 3), min(max(riz, 2), nz - 3)
+        res = []
+        for _ in range(2):  # a second run finds the first one's packets and planes
+            rec, snaps = s.forward_propagate_acoustic(v, w, six, siz, rix, riz, nz * nx < 1 << 20,
+                                                      interval)
+            res.append((rec, snaps))
+        for storage in ("all", "checkpoint"):
+            res.append(TSWRTMEngine(s, storage).migrate_shot(FloodModels(v, v, v2, 0, 0), w, six,
+                                                             siz, data, rix, riz, interval))
+        if nz * nx < 1 << 20:
+            fw = res[0][1]
+            img = np.ones((nz, nx), np.float32)
+            s.backward_propagate_and_correlate(v2, data, rix, riz, fw, img, interval)
+            res.append((img, None))
+        out.append(res)
+        s.close()
+    for a, b in zip(*out):
+        for x, y in zip(a, b):
+            if x is not None:
+                np.testing.assert_array_equal(x, y)
+    np.testing.assert_array_equal(out[0][0][0], out[0][1][0])
