@@ -18,6 +18,7 @@
 
 #include "arena.h"
 #include "batch_kernels.cuh"
+#include "resident.cuh"
 #include "small_kernels.cuh"
 #include "w2d_common.cuh"
 #include "wave2d_cuda.h"
@@ -46,6 +47,18 @@ struct HostShot {
     int mode = 0;            // 0: migration, 1: forward modelling
     int nt = 0, n_rec = 0;
     float* traces = nullptr;  // mode 1: (nt, n_rec)
+    // resident form: the cuts of this grid by number of CTAs (empty: step kernels), and the
+    // shot as that kernel takes it
+    std::vector<RsPlan> plans;
+    RsShot rs{};
+};
+
+// Shots that advance together in one resident launch, each with its cut.
+struct Wave {
+    std::vector<int> slots;
+    std::vector<RsPlan> plans;
+    int ctas = 0;
+    size_t item0 = 0;  // its first CTA in the item table
 };
 
 // Device copy of models shared by the shots submitted with one model key.
@@ -84,6 +97,15 @@ struct w2d_batch {
     int grid = 0;
     int form = 1;    // 1: one launch per phase step over all shots (grid form); 0: queue form
     int t_all = 0;   // tiles of the active shots (grid form launch size)
+    int n_step = 0;  // active shots that advance by step kernels (all, but for the waves')
+    // resident form: waves of the active set, their shots' records and CTAs, the packets
+    std::vector<Wave> waves;
+    RsShot* d_rs = nullptr;
+    int2* d_rs_items = nullptr;
+    size_t rs_items_cap = 0;
+    uint4* d_rs_x = nullptr;
+    size_t rs_x_cap = 0;
+    unsigned rs_tag = 0;
     cudaGraphExec_t gexec = nullptr;
     // grid form: the replay's launches as a graph, re-captured when the active set
     // (grid size, shot count) or the configuration changes
@@ -190,14 +212,14 @@ int capture_grid_replay(w2d_batch* b, int steps)
     a.shots = b->d_shots;
     a.maps = b->d_maps;
     a.items = b->d_items;
-    a.n_active = (int)b->active.size();
+    a.n_active = b->n_step;
     a.max_shots = b->max_shots;
     a.err = b->d_err;
     cudaGraph_t g = nullptr;
     W2D_CUDA_TRY(batch_step_attr_cfg(b));  // outside the capture
     W2D_CUDA_TRY(cudaStreamBeginCapture(b->st, cudaStreamCaptureModeThreadLocal));
     cudaError_t ce = cudaSuccess;
-    for (int j = 0; j < steps && ce == cudaSuccess; ++j) {
+    for (int j = 0; j < steps && b->n_step > 0 && ce == cudaSuccess; ++j) {
         a.j = j;
         ce = launch_step_cfg(b, a, j > 0 ? 1 : 0);
     }
@@ -310,6 +332,7 @@ int w2d_batch_create(w2d_batch** out, unsigned long long arena_bytes, int max_sh
         cudaMalloc(&b->d_prefix, sizeof(int) * (max_shots + 1)) != cudaSuccess ||
         cudaMalloc(&b->d_nact, sizeof(int)) != cudaSuccess ||
         cudaMalloc(&b->d_head, sizeof(unsigned)) != cudaSuccess ||
+        cudaMalloc(&b->d_rs, sizeof(RsShot) * max_shots) != cudaSuccess ||
         cudaMalloc(&b->d_err, sizeof(unsigned)) != cudaSuccess) {
         cudaGetLastError();
         set_error("table allocation failed");
@@ -338,7 +361,7 @@ void w2d_batch_destroy(w2d_batch* b)
     if (b->gexec_grid) cudaGraphExecDestroy(b->gexec_grid);
     for (void* p : {(void*)b->arena, (void*)b->d_shots, (void*)b->d_maps, (void*)b->d_active,
                     (void*)b->d_prefix, (void*)b->d_nact, (void*)b->d_head, (void*)b->d_err,
-                    (void*)b->d_items})
+                    (void*)b->d_items, (void*)b->d_rs, (void*)b->d_rs_items, (void*)b->d_rs_x})
         if (p) cudaFree(p);
     if (b->e0) cudaEventDestroy(b->e0);
     if (b->e1) cudaEventDestroy(b->e1);
@@ -650,8 +673,204 @@ int submit_job(w2d_batch* b, const w2d_shot_desc* d, int mode, int* slot_out)
     hsh.nt = nt;
     hsh.n_rec = n_rec;
     hsh.traces = h.traces;
+    bool one_per_column = true;
+    for (int i = 0; i < nx; ++i) one_per_column &= ptr[i + 1] - ptr[i] <= 1;
+    if (rs_lut_fits(hlut.data(), n_sp) &&
+        rs_shot_fits(nx, nz, d->src_ix, d->src_iz, n_rec, d->rec_iz, one_per_column)) {
+        hsh.plans = rs_plans(nx, nz, rs_capacity());
+        if (hsh.plans.empty() || !hsh.plans.back().ok()) hsh.plans.clear();
+        RsShot& r = hsh.rs;
+        r.nx = nx;
+        r.nz = nz;
+        r.ldx = ldx;
+        r.inv_dx2 = h.g.inv_dx2;
+        r.inv_dz2 = h.g.inv_dz2;
+        r.fs = h.g.free_surface;
+        r.n_sponge = n_sp;
+        r.lut = n_sp > 0 ? lut : nullptr;
+        r.src_ix = d->src_ix;
+        r.src_iz = d->src_iz;
+        r.rec_iz = d->rec_iz;
+        r.n_rec = n_rec;
+        r.rec_c0 = h.shot_ints[4];
+        r.rec_ptr = rptr;
+        r.rec_list = rlist;
+        r.nt = nt;
+        r.interval = interval;
+        for (int i = 0; i < n_waves; ++i) r.wave[i] = h.wave[i];
+        for (int i = 0; i < n_models; ++i) r.vel[i] = vel + (size_t)i * plane;
+        r.snaps = h.snaps;
+        r.n_snaps = (int)n_snaps;
+        r.plane = plane;
+        r.illum = h.illum;
+        r.image = h.image;
+        r.wavelet = wdev;
+        r.data = h.data;
+        r.rec_out = h.traces;
+        r.dt2_inj = h.dt2_inj;
+        r.img_dt = h.img_dt;
+        r.err = b->d_err;
+    }
     b->joining.push_back(slot);
     *slot_out = slot;
+    return W2D_OK;
+}
+
+// Waves of the active shots that run on chip.  A wave's step takes as long as its slowest
+// shot's; a tile that fills its SM does the most points per time.  So: as few waves as the
+// shots' smallest cuts need (largest first, each into the least loaded wave that has room),
+// then every wave's SMs shared out for the least step time of its slowest shot.
+std::vector<Wave> make_waves(const w2d_batch* b)
+{
+    std::vector<Wave> waves;
+    const int cap = rs_capacity();
+    auto least = [&](int slot) {
+        const std::vector<RsPlan>& p = b->hs[slot].plans;
+        int n = 1;
+        while (!p[n].ok()) ++n;
+        return n;
+    };
+    std::vector<std::pair<int, int>> need;  // smallest cut, slot
+    int total = 0;
+    for (int s : b->active)
+        if (!b->hs[s].plans.empty()) {
+            need.emplace_back(least(s), s);
+            total += need.back().first;
+        }
+    std::stable_sort(need.begin(), need.end(),
+                     [](const std::pair<int, int>& x, const std::pair<int, int>& y) {
+                         return x.first > y.first;
+                     });
+    if (!need.empty()) waves.resize((total + cap - 1) / cap);
+    for (const auto& q : need) {
+        Wave* w = nullptr;
+        for (Wave& c : waves)
+            if (c.ctas + q.first <= cap && (!w || c.ctas < w->ctas)) w = &c;
+        if (!w) {
+            waves.emplace_back();
+            w = &waves.back();
+        }
+        w->slots.push_back(q.second);
+        w->ctas += q.first;
+    }
+    waves.erase(std::remove_if(waves.begin(), waves.end(),
+                               [](const Wave& w) { return w.slots.empty(); }),
+                waves.end());
+    size_t item = 0;
+    for (Wave& w : waves) {
+        // the least time T for which every shot has a cut and the cuts fit together
+        auto ctas_at = [&](double T, std::vector<RsPlan>* out) {
+            int sum = 0;
+            for (int s : w.slots) {
+                const std::vector<RsPlan>& p = b->hs[s].plans;
+                int n = 1;
+                while (n < (int)p.size() && !(p[n].ok() && p[n].cost <= T)) ++n;
+                if (n == (int)p.size()) return cap + 1;
+                sum += p[n].ctas();
+                if (out) out->push_back(p[n]);
+            }
+            return sum;
+        };
+        double lo = 0.0, hi = 1.0;
+        for (int s : w.slots) hi = std::max(hi, b->hs[s].plans[least(s)].cost);
+        for (int i = 0; i < 24; ++i) {
+            const double mid = 0.5 * (lo + hi);
+            if (ctas_at(mid, nullptr) <= cap) hi = mid;
+            else lo = mid;
+        }
+        w.ctas = ctas_at(hi, &w.plans);
+        w.item0 = item;
+        item += w.ctas;
+    }
+    return waves;
+}
+
+template <typename T>
+int grow_table(w2d_batch* b, T** p, size_t* cap, size_t n)
+{
+    if (n <= *cap) return W2D_OK;
+    if (*p) {
+        W2D_CUDA_TRY(cudaStreamSynchronize(b->st));  // the last replay read it
+        cudaFree(*p);
+        *p = nullptr;
+        *cap = 0;
+    }
+    n = std::max<size_t>(1024, 2 * n);
+    if (cudaMalloc(p, n * sizeof(T)) != cudaSuccess) {
+        cudaGetLastError();
+        set_error("table allocation failed");
+        return W2D_ENOMEM;
+    }
+    *cap = n;
+    return W2D_OK;
+}
+
+// The waves' tables for a new active set.
+int upload_waves(w2d_batch* b)
+{
+    size_t n_items = 0, packets = 0;
+    for (const Wave& w : b->waves) {
+        size_t p = 0;
+        for (const RsPlan& c : w.plans) p += c.packets() * c.ctas();
+        packets = std::max(packets, p);
+        n_items += w.ctas;
+    }
+    if (n_items == 0) return W2D_OK;
+    int rc;
+    if ((rc = grow_table(b, &b->d_rs_items, &b->rs_items_cap, n_items))) return rc;
+    const size_t had = b->rs_x_cap;
+    if ((rc = grow_table(b, &b->d_rs_x, &b->rs_x_cap, packets))) return rc;
+    if (b->rs_x_cap != had) {
+        W2D_CUDA_TRY(cudaMemsetAsync(b->d_rs_x, 0, b->rs_x_cap * sizeof(uint4), b->st));
+        b->rs_tag = 0;
+    }
+    std::vector<int2> items;
+    items.reserve(n_items);
+    int rec = 0;
+    for (const Wave& w : b->waves)
+        for (const RsPlan& c : w.plans) {
+            for (int t = 0; t < c.ctas(); ++t) items.push_back(make_int2(rec, t));
+            ++rec;
+        }
+    W2D_CUDA_TRY(cudaMemcpyAsync(b->d_rs_items, items.data(), items.size() * sizeof(int2),
+                                 cudaMemcpyHostToDevice, b->st));
+    return W2D_OK;
+}
+
+// One replay of the waves: `steps` phase steps of each of their shots.
+int launch_waves(w2d_batch* b, int steps)
+{
+    if (b->rs_tag > 0x70000000u) {
+        W2D_CUDA_TRY(cudaMemsetAsync(b->d_rs_x, 0, b->rs_x_cap * sizeof(uint4), b->st));
+        b->rs_tag = 0;
+    }
+    std::vector<RsShot> recs;
+    for (const Wave& w : b->waves) {
+        uint4* x = b->d_rs_x;  // (the waves run one after another: they share it)
+        for (size_t i = 0; i < w.slots.size(); ++i) {
+            const HostShot& h = b->hs[w.slots[i]];
+            const RsPlan& c = w.plans[i];
+            RsShot r = h.rs;
+            r.gx = c.gx;
+            r.gz = c.gz;
+            r.maxc = c.maxc;
+            r.maxr = c.maxr;
+            r.k0 = h.k0;
+            r.k1 = std::min(h.k0 + steps, h.k_end);
+            r.xbuf = x;
+            r.tag0 = b->rs_tag;
+            x += c.packets() * c.ctas();
+            recs.push_back(r);
+        }
+        b->rs_tag += (unsigned)steps + 1u;
+    }
+    W2D_CUDA_TRY(cudaMemcpyAsync(b->d_rs, recs.data(), recs.size() * sizeof(RsShot),
+                                 cudaMemcpyHostToDevice, b->st));
+    for (const Wave& w : b->waves) {
+        W2D_CUDA_TRY(launch_acoustic_resident(recs[0], b->d_rs, b->d_rs_items + w.item0, w.ctas,
+                                              b->st));
+        b->last_launches++;
+    }
     return W2D_OK;
 }
 
@@ -692,6 +911,13 @@ int w2d_batch_launch(w2d_batch* b)
     if (b->active.empty()) return W2D_OK;
     int rc;
     if (b->active_dirty) {
+        b->waves.clear();
+        if (b->form == 1) b->waves = make_waves(b);
+        // the shots that advance by step kernels (the queue form: every shot)
+        std::vector<int> stepped;
+        for (int s : b->active)
+            if (b->form != 1 || b->hs[s].plans.empty()) stepped.push_back(s);
+        b->n_step = (int)stepped.size();
         std::vector<int> prefix(b->active.size() + 1, 0);
         for (size_t i = 0; i < b->active.size(); ++i)
             prefix[i + 1] = prefix[i] + b->h_shots[b->active[i]].ntiles;
@@ -702,45 +928,43 @@ int w2d_batch_launch(w2d_batch* b)
         W2D_CUDA_TRY(cudaMemcpyAsync(b->d_prefix, prefix.data(), (n + 1) * 4,
                                      cudaMemcpyHostToDevice, b->st));
         W2D_CUDA_TRY(cudaMemcpyAsync(b->d_nact, &n, 4, cudaMemcpyHostToDevice, b->st));
-        b->t_all = prefix[n];
+        b->t_all = 0;
         if (b->form == 1) {
-            // the grid form's work table: CTA r takes tile r - prefix[i] of active shot i
-            if ((size_t)b->t_all > b->items_cap) {
-                if (b->d_items) {
-                    W2D_CUDA_TRY(cudaStreamSynchronize(b->st));  // the last replay read it
-                    cudaFree(b->d_items);
-                    b->d_items = nullptr;
-                    b->items_cap = 0;
-                }
-                const size_t cap = std::max<size_t>(1024, 2 * (size_t)b->t_all);
-                W2D_CUDA_TRY(cudaMalloc(&b->d_items, cap * sizeof(int2)));
-                b->items_cap = cap;
+            // the grid form's work table: one CTA per tile of the stepped shots, in order
+            std::vector<int2> items;
+            for (int s : stepped)
+                for (int t = 0; t < b->h_shots[s].ntiles; ++t) items.push_back(make_int2(s, t));
+            b->t_all = (int)items.size();
+            const size_t had = b->items_cap;
+            if ((rc = grow_table(b, &b->d_items, &b->items_cap, items.size()))) return rc;
+            if (b->items_cap != had)
                 b->grid_key = -1;  // the captured replay holds the old table's address
-            }
-            std::vector<int2> items(b->t_all);
-            for (int i = 0; i < n; ++i)
-                for (int t = 0; t < prefix[i + 1] - prefix[i]; ++t)
-                    items[prefix[i] + t] = make_int2(b->active[i], t);
-            W2D_CUDA_TRY(cudaMemcpyAsync(b->d_items, items.data(), items.size() * sizeof(int2),
-                                         cudaMemcpyHostToDevice, b->st));
+            if (b->t_all)
+                W2D_CUDA_TRY(cudaMemcpyAsync(b->d_items, items.data(), items.size() * sizeof(int2),
+                                             cudaMemcpyHostToDevice, b->st));
+            if ((rc = upload_waves(b))) return rc;
         }
         b->active_dirty = false;
     }
     if (b->form == 1) {
-        // grid form: S * chunks launches, one phase step of every active shot each,
-        // then one advance of the shots' progress, replayed as one captured graph
+        // The waves of the shots that fit the chip; then S * chunks launches, one phase step
+        // of every other active shot each, and one advance of all shots' progress, replayed
+        // as one captured graph.  (20 gathers of 200-600 x 400-2000, 1500-3000 steps, host arrays in and out: 329 ms a
+        // batch with step kernels alone, 241 with waves; 20 shots of 150 x 400, 2000 steps: 53
+        // and 24.)
         const int steps = b->S * b->chunks;
         const long long key =
-            (((long long)b->t_all * 65536 + (long long)b->active.size()) * 4096 + steps) * 256 +
+            (((long long)b->t_all * 65536 + (long long)b->n_step) * 4096 + steps) * 256 +
             b->warps * 16 + b->rpw;
         if (b->grid_key != key || !b->gexec_grid) {
             if ((rc = capture_grid_replay(b, steps))) return rc;
             b->grid_key = key;
         }
         W2D_CUDA_TRY(cudaEventRecord(b->e0, b->st));
+        if (!b->waves.empty() && (rc = launch_waves(b, steps))) return rc;
         W2D_CUDA_TRY(cudaGraphLaunch(b->gexec_grid, b->st));
         W2D_CUDA_TRY(cudaEventRecord(b->e1, b->st));
-        b->last_launches = steps + 1;
+        b->last_launches += (b->n_step ? steps : 0) + 1;
         b->in_flight = true;
         return W2D_OK;
     }

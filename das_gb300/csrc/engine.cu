@@ -154,6 +154,7 @@ struct w2d_engine {
     // chip (no plan where it does not fit), and the packets its tiles exchange
     RsPlan rs;
     DevBuf<uint4> rs_x;
+    unsigned rs_tag = 0;  // the last tag used there
     DevBuf<int> rec_ptr, rec_list;
     DevBuf<float> wavelet, data, rec_out;
     DevBuf<float> snaps, ckpt;
@@ -471,10 +472,15 @@ RsShot rs_shot(w2d_engine* e)
 }
 
 // Phase steps [s.k0, s.k1) in one launch.
-int rs_run(w2d_engine* e, const RsShot& s)
+int rs_run(w2d_engine* e, RsShot& s)
 {
-    // no packet of an earlier launch may carry one of this launch's tags
-    W2D_CUDA_TRY(cudaMemsetAsync(e->rs_x.p, 0, e->rs.xbuf_bytes(), e->stream));
+    // no packet of an earlier launch carries one of this launch's tags
+    if (e->rs_tag > 0x70000000u) {
+        W2D_CUDA_TRY(cudaMemsetAsync(e->rs_x.p, 0, e->rs.xbuf_bytes(), e->stream));
+        e->rs_tag = 0;
+    }
+    s.tag0 = e->rs_tag;
+    e->rs_tag += (unsigned)(s.k1 - s.k0) + 1u;
     W2D_CUDA_TRY(launch_acoustic_resident(s, nullptr, nullptr, e->rs.ctas(), e->stream));
     e->last_launches++;
     return W2D_OK;
@@ -859,8 +865,10 @@ int w2d_engine_create(w2d_engine** out, int nx, int nz, float dx, float dz, doub
     cudaMemset(e->rec_ptr.p, 0, (nx + 1) * 4);
     if ((rc = ensure_tensor_maps(e))) return fail(rc);
     if (!e->use_arr && (!e->use_lut || lut_ok)) {
-        e->rs = rs_plan(nx, nz, rs_capacity());
-        if (e->rs.ok() && (rc = e->rs_x.ensure(e->rs.xbuf_bytes() / sizeof(uint4)))) return fail(rc);
+        e->rs = rs_plans(nx, nz, rs_capacity()).back();
+        if (e->rs.ok() && ((rc = e->rs_x.ensure(e->rs.xbuf_bytes() / sizeof(uint4))) ||
+                           cudaMemset(e->rs_x.p, 0, e->rs.xbuf_bytes()) != cudaSuccess))
+            return fail(rc ? rc : W2D_ECUDA);
     }
     if (cudaDeviceSynchronize() != cudaSuccess) {
         set_error("engine set-up failed");

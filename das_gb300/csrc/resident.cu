@@ -770,7 +770,7 @@ static __global__ void __launch_bounds__(RS_T, 1)
             // nothing derived from the records or from m is kept from step to step: it
             // would not fit the registers
             asm volatile("" : "+r"(m.e), "+r"(m.i), "+r"(m.b)::"memory");
-            const unsigned tag = (unsigned)(k - s.k0) + 1u;
+            const unsigned tag = s.tag0 + (unsigned)(k - s.k0) + 1u;
             const int it = fwd ? k : 2 * nt - 1 - k;
             const int cur = t.plane[par], nxt = t.plane[par ^ 1];
             if (!halo) {

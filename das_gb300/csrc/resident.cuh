@@ -3,6 +3,7 @@
 #pragma once
 
 #include <algorithm>
+#include <vector>
 
 #include "w2d_common.cuh"
 
@@ -40,12 +41,14 @@ struct RsShot {
     float dt2_inj, img_dt;
     float minus_zero = -0.0f;  // an operand the compiler must not know (see mul2)
     uint4* xbuf;               // packets: tile, slot, {left, right, top, bottom}
+    unsigned tag0;             // the launch's tags are tag0 + 1 ..: none was used in xbuf before
     unsigned* err;
 };
 
 // ---- host: how a grid is cut -------------------------------------------------------
 struct RsPlan {
     int gx = 0, gz = 0, maxc = 0, maxr = 0;
+    double cost = 0;  // estimated cycles of a step
     bool ok() const { return gx > 0; }
     int ctas() const { return gx * gz; }
     size_t packets() const { return 2 * (size_t)(2 * maxr + 8 * maxc); }  // of one tile
@@ -73,14 +76,13 @@ __host__ __device__ inline void rs_interior(int nrows, int ncol, int* nci, int* 
     *nseg = (ni + *R - 1) / *R;
 }
 
-// The cut of an nx x nz grid into at most max_ctas tiles with the least estimated step
-// time: what a step costs is its slowest tile, so columns and rows are split evenly and
-// the estimate (in cycles) is that of the largest tile.  No plan when the grid does not
-// fit the SMs' shared memory.
-inline RsPlan rs_plan(int nx, int nz, int max_ctas)
+// The cuts of an nx x nz grid: element n is the one into at most n tiles (n = 1 ..
+// max_ctas) with the least estimated step time, none where the grid does not fit the
+// shared memory of n SMs.  What a step costs is its slowest tile, so columns and rows are
+// split evenly and the estimate (in cycles) is that of the largest tile.
+inline std::vector<RsPlan> rs_plans(int nx, int nz, int max_ctas)
 {
-    RsPlan best;
-    double best_cost = 1e30;
+    std::vector<RsPlan> best(std::max(max_ctas, 0) + 1);
     const int w4 = (nx + 3) / 4;
     for (int gx = 1; gx <= max_ctas && (gx == 1 || w4 / gx >= 2); ++gx)
         for (int gz = 1; gx * gz <= max_ctas && (gz == 1 || nz / gz >= 4); ++gz) {
@@ -93,16 +95,18 @@ inline RsPlan rs_plan(int nx, int nz, int max_ctas)
             if (R > RS_MAXR) continue;
             const double warps = std::max(1.0, nci * nseg / 32.0);
             const double inner = R ? (R + 1.5) * std::max(warps / 4 * 75.0, 150.0) : 0.0;
-            const double cost = 600.0 + ne / 128.0 * 110.0 + inner +
-                                std::max(0.0, 1200.0 - inner) + 0.5 * gx * gz;
-            if (cost < best_cost) {
-                best_cost = cost;
-                best.gx = gx;
-                best.gz = gz;
-                best.maxc = ncol;
-                best.maxr = nrows;
-            }
+            const double cost = 600.0 + ne / 128.0 * 110.0 + inner + std::max(0.0, 1200.0 - inner);
+            RsPlan& b = best[gx * gz];
+            if (b.ok() && b.cost <= cost) continue;
+            b.gx = gx;
+            b.gz = gz;
+            b.maxc = ncol;
+            b.maxr = nrows;
+            b.cost = cost;
         }
+    for (int n = 1; n <= max_ctas; ++n)
+        if (!best[n].ok() || (best[n - 1].ok() && best[n - 1].cost <= best[n].cost))
+            best[n] = best[n - 1];
     return best;
 }
 

@@ -66,3 +66,47 @@ def test_resident_equals_steps(nz, nx, fs, n_sponge, riz, kind, interval, nt):
             if x is not None:
                 np.testing.assert_array_equal(x, y)
     np.testing.assert_array_equal(out[0][0][0], out[0][1][0])
+
+
+def test_batch_waves_equal_steps():
+    """A batch whose shots advance on chip, several to a launch and over more than one
+    launch, beside shots that keep the step kernels; modelling jobs among them."""
+    from das_gb300.batch import BatchEngine, ModelJob, ShotJob
+    from das_gb300.rtm_engine import TSWRTMEngine
+    from das_gb300.velocity_flood import FloodModels
+    from das_gb300.wave_solver import WaveSolver2D
+    rng = np.random.default_rng(7)
+    dx, dt, jobs = 5.0, 5e-4, []
+    for k, (nz, nx, nt) in enumerate([(90, 260, 150), (600, 2000, 70), (33, 77, 64), (500, 1900, 90),
+                                      (128, 301, 180), (1024, 4100, 20), (590, 1990, 75),
+                                      (61, 130, 333)]):
+        v = rng.uniform(1500, 3200, (nz, nx)).astype(np.float32)
+        w = rng.standard_normal(nt).astype(np.float32)
+        rix = np.arange(nx) if k % 2 else rng.permutation(nx)[: nx // 2]
+        if k == 4:
+            rix = np.zeros(9, int) + 5  # one column: the step kernels
+        if k == 6:
+            jobs.append(ModelJob(nx, nz, dx, dx, dt, v, w, rix, nx // 2, 2))
+            continue
+        data = rng.standard_normal((nt, len(rix))).astype(np.float32)
+        jobs.append(ShotJob(nx, nz, dx, dx, dt, v, v * np.float32(1.01), w, data, rix, nx // 2, 2, 2,
+                            1 + k % 3, 10 if k else -1, 0.0015, k != 2))
+    eng = BatchEngine(arena_bytes=8 << 30, max_shots=16, tile=(4, 4), steps_per_launch=8,
+                      launches_per_graph=3)
+    for _ in range(2):
+        results, _ = eng.run(jobs)
+        for j, r in zip(jobs, results):
+            s = WaveSolver2D(j.nx, j.nz, dx, dx, dt, max(j.n_sponge, 0), 0.0015, j.free_surface_top)
+            s.set_launch("grid", False)
+            if isinstance(j, ModelJob):
+                rec, _ = s.forward_propagate_acoustic(j.vel, j.wavelet, j.source_ix, 2,
+                                                      j.receiver_ix, 2)
+                np.testing.assert_array_equal(r, rec)
+            else:
+                img, ill = TSWRTMEngine(s, "all").migrate_shot(
+                    FloodModels(j.vel_fwd, j.vel_fwd, j.vel_bwd, 0, 0), j.wavelet, j.source_ix, 2,
+                    j.data, j.receiver_ix, 2, j.snapshot_interval)
+                np.testing.assert_array_equal(r[0], img)
+                np.testing.assert_array_equal(r[1], ill)
+            s.close()
+    eng.close()
