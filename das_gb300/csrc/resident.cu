@@ -24,8 +24,10 @@
 //     rows), one per thread.  They are computed first and published to the neighbours
 //     at once, so that the exchange runs while
 //   * phase I computes the other units: a thread owns one column of units over up to
-//     RS_MAXR consecutive rows, with a five-row register window along z and the x
-//     neighbours from the adjacent lanes by shuffles.
+//     RS_MAXR consecutive rows, with a five-row register window along z.  (The x
+//     neighbours come from shared memory: as register pairs, ready for the packed
+//     arithmetic; from the adjacent lanes, by shuffles and selects, they cost ten more
+//     instructions of a hundred.)
 //   * The halo warp collects the neighbours' edges meanwhile into the halo of p_next,
 //     stages the next step's injection values, and prefetches the next snapshot into L2.
 // One barrier ends the step.
@@ -185,23 +187,25 @@ __device__ __forceinline__ RsPacket rs_peek(const uint4* p)
 }
 
 // One step of four points: reference operation order, every operation rounded.
-// e: the two points left (l2, l1) and right (r1, r2) of c; w0, w1, w3, w4: rows z-2..z+2.
+// l, r: the two points left and right of c; w0, w1, w3, w4: rows z-2..z+2.
 struct RsConst {
     f32x2 k0, k1, k2, dx2, dz2, m2, z;
 };
 __device__ __forceinline__ F4 rs_stencil(const RsConst& k, const F4& w0, const F4& w1, const F4& c,
-                                         const F4& w3, const F4& w4, float l2, float l1, float r1,
-                                         float r2, const F4& pp, const F4& v)
+                                         const F4& w3, const F4& w4, f32x2 l, f32x2 r,
+                                         const F4& pp, const F4& v)
 {
-    float cx, cy, cz, cw;
+    float cx, cy, cz, cw, l2, l1, r1, r2;
+    upk(l, l2, l1);
+    upk(r, r1, r2);
     upk(c.a, cx, cy);
     upk(c.b, cz, cw);
     auto mul = [&](f32x2 a, f32x2 b) { return mul2(a, b, k.z); };
     const f32x2 kca = mul(k.k0, c.a), kcb = mul(k.k0, c.b);
     // (c2*(m2+p2) + c1*(m1+p1)) + c0*c along x, then along z
-    const f32x2 xa = mul(add2(add2(mul(k.k2, add2(pk(l2, l1), c.b)),
+    const f32x2 xa = mul(add2(add2(mul(k.k2, add2(l, c.b)),
                                    mul(k.k1, pk(fadd(l1, cy), fadd(cx, cz)))), kca), k.dx2);
-    const f32x2 xb = mul(add2(add2(mul(k.k2, add2(c.a, pk(r1, r2))),
+    const f32x2 xb = mul(add2(add2(mul(k.k2, add2(c.a, r)),
                                    mul(k.k1, pk(fadd(cy, cw), fadd(cz, r1)))), kcb), k.dx2);
     const f32x2 za = mul(add2(add2(mul(k.k2, add2(w0.a, w4.a)), mul(k.k1, add2(w1.a, w3.a))),
                               kca), k.dz2);
@@ -226,6 +230,7 @@ struct RsTile {
     int hx;                          // float2 [parity][side][row]: columns beside the tile
     int inj;                         // [parity][pitch]: added to the receiver row
     int injs;                        // [parity]: added to the source cell
+    int pre;                         // [parity]: the source cell before that
     int ring;                        // [3][4]: never-written cells of the receiver row
     int fx, fz;                      // sponge by column, by row
     int rk;                          // receiver of a column, -1: none
@@ -234,6 +239,7 @@ struct RsTile {
     int half, in;                    // packets of one slot; where this tile's begin
     int nci, nseg, R;                // phase I: columns, segments, rows of a segment
     int tm;                          // tensor-memory address
+    int next;                        // [parity]: groups of packets taken
     float dx2, dz2;
     float z;                         // -0
 };
@@ -241,63 +247,75 @@ static_assert(sizeof(RsTile) <= RS_TILE_FLOATS * 4 && sizeof(RsShot) <= RS_SHOT_
                   sizeof(RsShot) % 4 == 0,
               "the tile's and the shot's records fit their places");
 
+constexpr int RS_PLANE0 = RS_TILE_FLOATS + RS_SHOT_FLOATS;  // where the first plane begins
+
 extern __shared__ __align__(128) float rs_smem[];
 __device__ __forceinline__ const RsTile& rs_tile() { return *reinterpret_cast<RsTile*>(rs_smem); }
-__device__ __forceinline__ float2 rs_f2(int o) { return *reinterpret_cast<float2*>(rs_smem + o); }
+__device__ __forceinline__ f32x2 rs_pair(int o) { return *reinterpret_cast<f32x2*>(rs_smem + o); }
 
 // Which of the four never-written cells of a row column ix is.
 __device__ __forceinline__ int rs_cell(int ix, int nx) { return ix < 2 ? ix : 4 + ix - nx; }
 
 // The rules of the receiver row, the source row and the free surface for the unit at
 // column c of a row, whose new values are u (zero on never-written columns: those not in
-// xm).  par: parity of the staged injection; nb: which of the three rotating buffers
-// p_next is.  Sampling sees the value before the next step's injection.
+// xm).  par: parity of the step; nb: which of the three rotating buffers p_next is.
+// (Receivers are sampled by the halo warp, from p_curr of the next step: this is on the
+// way from a tile's edge to its neighbours.)
 __device__ __forceinline__ F4 rs_special(const F4& v, int nxt, int row, int c, int par, int nb,
-                                         unsigned xm, float* rec_out, bool inject)
+                                         unsigned xm, int pitch, bool inject)
 {
     const RsTile& t = rs_tile();
+    const int rec_row = t.rec_row, src_row = t.src_row, mirror = t.mirror, inj = t.inj;
     float u[4];
     f4_get(v, u);
-    const bool at_rec = row == t.rec_row;
-    const int ix = t.x0 + 4 * c;
+    const bool at_rec = row == rec_row && inject;
     float* ring = rs_smem + t.ring + 4 * nb;
-    if (at_rec && xm != 15u) {
+    float4 d = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (at_rec) d = *reinterpret_cast<const float4*>(rs_smem + inj + par * pitch + 4 * c);
+    const int ix = t.x0 + 4 * c;
+    if (row == rec_row && xm != 15u) {
 #pragma unroll
         for (int j = 0; j < 4; ++j)
             if (!((xm >> j) & 1u) && ix + j < t.nx) u[j] = ring[rs_cell(ix + j, t.nx)];
     }
-    if (row == t.mirror)  // p_next[1,:] = -p_next[2,:] over every column
-        *reinterpret_cast<float4*>(rs_smem + nxt + (row + 1) * t.pitch + 4 * c) =
+    if (row == mirror)  // p_next[1,:] = -p_next[2,:] over every column
+        *reinterpret_cast<float4*>(rs_smem + nxt + (row + 1) * pitch + 4 * c) =
             make_float4(-u[0], -u[1], -u[2], -u[3]);
     if (at_rec) {
-        if (rec_out) {
-            const int4 r = *reinterpret_cast<const int4*>(rs_smem + t.rk + 4 * c);
-            if (r.x >= 0) rec_out[r.x] = u[0];
-            if (r.y >= 0) rec_out[r.y] = u[1];
-            if (r.z >= 0) rec_out[r.z] = u[2];
-            if (r.w >= 0) rec_out[r.w] = u[3];
-        }
-        if (inject) {
-            const float4 d =
-                *reinterpret_cast<const float4*>(rs_smem + t.inj + par * t.pitch + 4 * c);
-            u[0] = fadd(u[0], d.x);
-            u[1] = fadd(u[1], d.y);
-            u[2] = fadd(u[2], d.z);
-            u[3] = fadd(u[3], d.w);
-            if (xm != 15u) {
+        u[0] = fadd(u[0], d.x);
+        u[1] = fadd(u[1], d.y);
+        u[2] = fadd(u[2], d.z);
+        u[3] = fadd(u[3], d.w);
+        if (xm != 15u) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    if (!((xm >> j) & 1u) && ix + j < t.nx) ring[rs_cell(ix + j, t.nx)] = u[j];
-            }
+            for (int j = 0; j < 4; ++j)
+                if (!((xm >> j) & 1u) && ix + j < t.nx) ring[rs_cell(ix + j, t.nx)] = u[j];
         }
     }
-    if (row == t.src_row && c == t.src_x >> 2) {
+    if (row == src_row && c == t.src_x >> 2) {
         const float w = rs_smem[t.injs + par];
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-            if (j == (t.src_x & 3)) u[j] = fadd(u[j], w);
+            if (j == (t.src_x & 3)) {
+                rs_smem[t.pre + par] = u[j];
+                u[j] = fadd(u[j], w);
+            }
     }
     return f4_of(u);
+}
+
+// Receiver samples of the step whose p_next is now the plane at pl: row[r] for every
+// receiver r of the tile (the whole warp).  par: parity of that step.
+__device__ __forceinline__ void rs_sample(float* row, int pl, int par)
+{
+    const RsTile& t = rs_tile();
+    const int src_x = t.src_row == t.rec_row ? t.src_x : -1;
+    for (int c = threadIdx.x & 31; c < t.pitch; c += 32) {
+        const int r = __float_as_int(rs_smem[t.rk + c]);
+        float v = rs_smem[pl + (t.rec_row + 2) * t.pitch + c];
+        if (c == src_x) v = rs_smem[t.pre + par];  // without the next step's injection
+        if (r >= 0) row[r] = v;
+    }
 }
 
 // Pointwise work of a fused step on one unit of p_curr: snapshot copy and illumination
@@ -339,7 +357,7 @@ __device__ __forceinline__ F4 rs_frame(const F4& u, const float4& fx, float fz, 
 // leaves next to no L1): the rest is read from the tile's record.
 struct RsMine {
     // edge unit: row, unit column << 16, and whether there is one (bit 31), it is written
-    // (bit 30), and a rule of its own applies (bit 29); packets it sends along x and z,
+    // (bit 30), a rule of its own applies (bit 29), it is the last column's (bit 28); packets it sends along x and z,
     // as indices into the packet buffer, -1: none
     unsigned e;
     int ox, oz;
@@ -349,6 +367,8 @@ struct RsMine {
     // edge unit (bits 16-19) and of the interior units (bits 20-23), and whether the warp's
     // interior units (bit 24) or edge units (bit 25) meet the sponge or the edge columns
     unsigned b;
+    unsigned h;           // edge column: its cells beside the tile in RsTile::hx, and (above
+                          // bit 16) how far the other parity's are
     uint32_t tm;          // tensor-memory address of this thread's words
 
     __device__ __forceinline__ int er() const { return e & 0xffff; }
@@ -356,6 +376,7 @@ struct RsMine {
     __device__ __forceinline__ bool e_live() const { return e >> 31; }
     __device__ __forceinline__ bool e_write() const { return (e >> 30) & 1u; }
     __device__ __forceinline__ bool e_spec() const { return (e >> 29) & 1u; }
+    __device__ __forceinline__ bool last_col() const { return (e >> 28) & 1u; }
     __device__ __forceinline__ int c() const { return i & 0xff; }
     __device__ __forceinline__ int r0() const { return (i >> 8) & 0xffff; }
     __device__ __forceinline__ int n() const { return i >> 24; }
@@ -364,6 +385,10 @@ struct RsMine {
     __device__ __forceinline__ unsigned i_xm() const { return (b >> 20) & 15u; }
     __device__ __forceinline__ bool i_frame() const { return (b >> 24) & 1u; }
     __device__ __forceinline__ bool e_frame() const { return (b >> 25) & 1u; }
+    __device__ __forceinline__ int hx(int par) const
+    {
+        return (int)(h & 0xffffu) + (par ? (int)(h >> 16) : 0);
+    }
 };
 static_assert(RS_MAXR <= 15, "rows with a rule: 15 bits");
 
@@ -376,13 +401,12 @@ struct RsFused {
 
 // Phase I of one step: rows of one unit column.  FUSED: see RsFused.
 template <bool FUSED>
-__device__ __forceinline__ void rs_inner(const RsMine& m, const RsConst& k, int cur, int nxt,
-                                         int R, const RsFused& fu, f32x2 img_dt)
+__device__ __forceinline__ void rs_inner(const RsMine& m, const RsConst& k, int pitch, int cur,
+                                         int nxt, int R, const RsFused& fu, f32x2 img_dt)
 {
     const RsTile& t = rs_tile();
     const bool frame = m.i_frame();
-    const int pitch = t.pitch, lane = threadIdx.x & 31, c = m.c(), r0 = m.r0(), n = m.n();
-    const bool lds_l = lane == 0 || c == 1, lds_r = lane == 31 || c == t.ncol - 2;
+    const int c = m.c(), r0 = m.r0(), n = m.n();
     // addresses advance by rows and stay on the thread's last one
     int oc = cur + (r0 + 2) * pitch + 4 * c;
     const int dn = nxt - cur;
@@ -390,7 +414,7 @@ __device__ __forceinline__ void rs_inner(const RsMine& m, const RsConst& k, int 
        w2 = ld_f4(rs_smem + oc), w3 = ld_f4(rs_smem + oc + pitch);
     float4 fx = make_float4(1.f, 1.f, 1.f, 1.f);
     if (frame) fx = *reinterpret_cast<const float4*>(rs_smem + t.fx + 4 * c);
-    const int ofz = t.fz + r0;
+    const int ofz = frame ? t.fz + r0 : 0;
     uint32_t cb[4], ab[4];
     tm_ld4(m.tm + RS_TM_C, cb);
     size_t goff = 0;
@@ -420,23 +444,8 @@ __device__ __forceinline__ void rs_inner(const RsMine& m, const RsConst& k, int 
             f2 = __ldcs(reinterpret_cast<const float4*>(fu.snap_in + goff + 2 * (size_t)t.ldx));
         const F4 w4 = ld_f4(rs_smem + oc + 2 * pitch);
         const F4 pp = ld_f4(rs_smem + oc + dn);
-        float c4[4];
-        f4_get(w2, c4);
-        float l2 = __shfl_up_sync(0xffffffffu, c4[2], 1);
-        float l1 = __shfl_up_sync(0xffffffffu, c4[3], 1);
-        float r1 = __shfl_down_sync(0xffffffffu, c4[0], 1);
-        float r2 = __shfl_down_sync(0xffffffffu, c4[1], 1);
-        if (lds_l) {
-            const float2 e = rs_f2(oc - 2);
-            l2 = e.x;
-            l1 = e.y;
-        }
-        if (lds_r) {
-            const float2 e = rs_f2(oc + 4);
-            r1 = e.x;
-            r2 = e.y;
-        }
-        F4 u = rs_stencil(k, w0, w1, w2, w3, w4, l2, l1, r1, r2, pp, v);
+        const f32x2 l = rs_pair(oc - 2), r = rs_pair(oc + 4);
+        F4 u = rs_stencil(k, w0, w1, w2, w3, w4, l, r, pp, v);
         if (frame) u = rs_frame(u, fx, rs_smem[ofz + (ok ? i : 0)], m.i_xm(), k.z);
         if (ok) st_f4(rs_smem + oc + dn, u);
         if (FUSED) {
@@ -461,26 +470,36 @@ __device__ __forceinline__ void rs_inner(const RsMine& m, const RsConst& k, int 
     if (FUSED && fu.acc) tm_wait_st();
 }
 
-// The halo warp: this step's packets (at src) into the halo of p_next.  False: a wait
-// gave up (recorded), or another CTA's did.
+// This step's packets (at src) into the halo of p_next, FLIGHT groups of 32 at a time: the
+// halo warp from the start of the step, and every compute warp that is done with its units
+// takes its share of what is left (next: the step's counter of groups taken).  False: a
+// wait gave up (recorded), or another CTA's did.  (Looking at a sample of the packets
+// before all of them are looked at measured slower: one more round trip, 2.0 -> 2.3 us a
+// step at 150 x 400, 7.7 -> 8.3 at 1000 x 4000.)
+template <int FLIGHT>
 __device__ __forceinline__ bool rs_collect(const uint4* src, unsigned tag, int nxt, int par,
-                                           unsigned* err)
+                                           int next, unsigned* err)
 {
     const RsTile& t = rs_tile();
-    const int nL = t.n_l, nLR = t.n_lr, nLRT = t.n_lrt, n_in = t.n_in;
-    // left, right: rows of hx; upper, lower: the plane's halo rows
-    const int oL = t.hx + 4 * par * t.nrows, oR = oL + 2 * (t.nrows - nL), oT = nxt - 2 * nLR,
-              oB = nxt + (t.nrows + 2) * t.pitch - 2 * nLRT;
-    for (int b0 = threadIdx.x & 31; b0 < n_in; b0 += 32 * RS_FLIGHT) {
+    const int n_in = t.n_in, lane = threadIdx.x & 31;
+    for (;;) {
+        int g = 0;
+        if (lane == 0) g = atomicAdd(reinterpret_cast<int*>(rs_smem + next), FLIGHT);
+        const int b0 = 32 * __shfl_sync(0xffffffffu, g, 0) + lane;
+        if (b0 - lane >= n_in) return true;
         unsigned left = 0;
 #pragma unroll
-        for (int j = 0; j < RS_FLIGHT; ++j) left |= b0 + 32 * j < n_in ? 1u << j : 0u;
+        for (int j = 0; j < FLIGHT; ++j) left |= b0 + 32 * j < n_in ? 1u << j : 0u;
         for (int tries = 0; left; ++tries) {
-            RsPacket v[RS_FLIGHT];  // (those that came already are looked at again)
+            RsPacket v[FLIGHT];  // (unconditionally: partly loaded, they would spill)
 #pragma unroll
-            for (int j = 0; j < RS_FLIGHT; ++j) v[j] = rs_peek(src + min(b0 + 32 * j, n_in - 1));
+            for (int j = 0; j < FLIGHT; ++j) v[j] = rs_peek(src + min(b0 + 32 * j, n_in - 1));
+            // left, right: rows of hx; upper, lower: the plane's halo rows
+            const int nL = t.n_l, nLR = t.n_lr, nLRT = t.n_lrt;
+            const int oL = t.hx + 4 * par * t.nrows, oR = oL + 2 * (t.nrows - nL),
+                      oT = nxt - 2 * nLR, oB = nxt + (t.nrows + 2) * t.pitch - 2 * nLRT;
 #pragma unroll
-            for (int j = 0; j < RS_FLIGHT; ++j)
+            for (int j = 0; j < FLIGHT; ++j)
                 if (((left >> j) & 1u) && (unsigned)(v[j].a >> 32) == tag &&
                     (unsigned)(v[j].b >> 32) == tag) {
                     const int i = b0 + 32 * j;
@@ -491,15 +510,16 @@ __device__ __forceinline__ bool rs_collect(const uint4* src, unsigned tag, int n
                     left &= ~(1u << j);
                 }
             if (left && (tries & 1023) == 1023) {
-                if (*reinterpret_cast<volatile unsigned*>(err) & ERR_ABORT) return false;
-                if (tries >= RS_POLLS) {
+                bool stop = *reinterpret_cast<volatile unsigned*>(err) & ERR_ABORT;
+                if (!stop && tries >= RS_POLLS) {
                     atomicOr(err, ERR_DEP_TIMEOUT | ERR_ABORT);
-                    return false;
+                    stop = true;
                 }
+                if (stop) break;
             }
         }
+        if (__any_sync(0xffffffffu, left)) return false;
     }
-    return true;
 }
 
 // many: the launch covers several shots, items[CTA] = {shot, tile}; else the one shot.
@@ -538,7 +558,7 @@ static __global__ void __launch_bounds__(RS_T, 1)
         w.pitch = pitch;
         w.left = tx > 0;
         w.right = tx < gx - 1;
-        int sp = RS_TILE_FLOATS + RS_SHOT_FLOATS;
+        int sp = RS_PLANE0;
         auto place = [&](int floats) {
             const int o = sp;
             sp += floats;
@@ -553,7 +573,9 @@ static __global__ void __launch_bounds__(RS_T, 1)
         w.fz = place((nrows + 3) / 4 * 4);
         w.ring = place(12);
         w.injs = place(2);
+        w.pre = place(2);
         w.tm = place(1);
+        w.next = place(2);
         w.dx2 = s.inv_dx2;
         w.dz2 = s.inv_dz2;
         w.z = s.minus_zero;
@@ -640,11 +662,13 @@ static __global__ void __launch_bounds__(RS_T, 1)
         };
         const bool e_write = e_live && w.z0 + er >= 2 && w.z0 + er < nz - 2;
         m.e = (unsigned)er | (unsigned)ec << 16 | (unsigned)e_live << 31 |
-              (unsigned)e_write << 30 | (unsigned)(e_write && has_rule(er, ec)) << 29;
+              (unsigned)e_write << 30 | (unsigned)(e_write && has_rule(er, ec)) << 29 |
+              (unsigned)(ec == ncol - 1) << 28;
         const bool live = !halo && tid < w.nci * w.nseg;
         const int seg = live ? tid / w.nci : 0;
         const int ic = live ? 1 + tid - seg * w.nci : 1, r0 = 2 + seg * w.R;
         const int n_rows = live ? min(w.R, nrows - 2 - r0) : 0;
+        m.h = (unsigned)(w.hx + 2 * er + (ec == 0 ? 0 : 2 * nrows)) | (unsigned)(4 * nrows) << 16;
         m.i = (unsigned)ic | (unsigned)r0 << 8 | (unsigned)n_rows << 24;
         m.b = 0;
         for (int i = 0; i < n_rows; ++i) m.b |= has_rule(r0 + i, ic) ? 1u << i : 0u;
@@ -680,6 +704,8 @@ static __global__ void __launch_bounds__(RS_T, 1)
     kc.m2 = pk(-2.0f, -2.0f);
     kc.z = pk(t.z, t.z);
     bool bad = false;
+    unsigned tag = s.tag0 + 1u;
+    const int pitch = t.pitch, dpl = t.plane[1] - t.plane[0];
 
     for (int ka = s.k0; ka < s.k1 && !bad;) {
         // the steps of one pass
@@ -698,6 +724,9 @@ static __global__ void __launch_bounds__(RS_T, 1)
             const int it = 2 * nt - 1 - k;
             return !fwd && it >= 1 && t.rec_row >= 0 ? s.data + (size_t)(it - 1) * s.n_rec
                                                      : nullptr;
+        };
+        auto rec_row_out = [&](int k) {
+            return fwd && s.rec_out ? s.rec_out + (size_t)k * s.n_rec : nullptr;
         };
         auto rec_of = [&](int c) { return __float_as_int(rs_smem[t.rk + c]); };
         // ---- the state into the SM
@@ -726,6 +755,7 @@ static __global__ void __launch_bounds__(RS_T, 1)
                 hx[nrows + r] = g;
                 hx[2 * nrows + r] = hx[3 * nrows + r] = make_float2(0.f, 0.f);
             }
+            if (tid < 2) rs_smem[t.next + tid] = __int_as_float(0);
             if (tid < 12) {
                 const int b = tid >> 2, cell = tid & 3;
                 const int ix = cell < 2 ? cell : t.nx - 4 + cell;
@@ -770,90 +800,97 @@ static __global__ void __launch_bounds__(RS_T, 1)
             // nothing derived from the records or from m is kept from step to step: it
             // would not fit the registers
             asm volatile("" : "+r"(m.e), "+r"(m.i), "+r"(m.b)::"memory");
-            const unsigned tag = s.tag0 + (unsigned)(k - s.k0) + 1u;
-            const int it = fwd ? k : 2 * nt - 1 - k;
-            const int cur = t.plane[par], nxt = t.plane[par ^ 1];
+            const int cur = RS_PLANE0 + (par ? dpl : 0), nxt = RS_PLANE0 + (par ? 0 : dpl);
+            const bool on = rem == 0;  // a step with a snapshot
             if (!halo) {
-                RsFused fu{nullptr, nullptr, false};
-                if (rem == 0 && s.snaps) {
-                    float* sn = s.snaps + (size_t)(ks - s.slot0) * s.plane;
-                    if (fwd) fu.snap_out = sn;
-                    else if (s.image && ks < s.n_snaps) fu.snap_in = sn;
-                }
-                fu.acc = fwd ? rem == 0 && s.illum : fu.snap_in != nullptr;
-                const bool fused = fu.acc || fu.snap_out;
-                const int nb = m3 == 0 ? 2 : m3 - 1;
-                float* rec_out = fwd && s.rec_out ? s.rec_out + (size_t)it * s.n_rec : nullptr;
-                const bool inject = !fwd && it >= 1;
                 // ---- phase E
                 if (e_warp) {
-                    const int pitch = t.pitch, er = m.er(), ec = m.ec();
-                    const size_t eo = (size_t)(t.z0 + er) * t.ldx + t.x0 + 4 * ec;
-                    uint32_t cb[4], ab[4];
+                    const int ec = m.ec(), oc = cur + (m.er() + 2) * pitch + 4 * ec;
+                    uint32_t cb[4];
                     tm_converge();
                     tm_ld4(m.tm + RS_TM_CE, cb);
-                    if (fu.acc) tm_ld4(m.tm + RS_TM_AE, ab);
-                    float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (fu.snap_in && m.e_live())
-                        f = __ldcs(reinterpret_cast<const float4*>(fu.snap_in + eo));
-                    const int oc = cur + (er + 2) * pitch + 4 * ec;
                     const F4 c = ld_f4(rs_smem + oc);
-                    const float2 l = rs_f2(ec > 0 ? oc - 2 : t.hx + 4 * par * t.nrows + 2 * er);
-                    const float2 g = rs_f2(ec < t.ncol - 1
-                                               ? oc + 4
-                                               : t.hx + (4 * par + 2) * t.nrows + 2 * er);
+                    const f32x2 l = rs_pair(ec > 0 ? oc - 2 : m.hx(par)),
+                                r = rs_pair(m.last_col() ? m.hx(par) : oc + 4);
                     const F4 w0 = ld_f4(rs_smem + oc - 2 * pitch), w1 = ld_f4(rs_smem + oc - pitch),
                              w3 = ld_f4(rs_smem + oc + pitch),
                              w4 = ld_f4(rs_smem + oc + 2 * pitch);
                     float* np = rs_smem + oc + nxt - cur;
                     const F4 pp = ld_f4(np);
-                    if (fu.acc) tm_wait_ld2(cb, ab);
-                    else tm_wait_ld(cb);
-                    F4 u = rs_stencil(kc, w0, w1, c, w3, w4, l.x, l.y, g.x, g.y, pp, f4_bits(cb));
+                    uint4* out = s.xbuf + (tag & 1u) * t.half;
+                    tm_wait_ld(cb);
+                    F4 u = rs_stencil(kc, w0, w1, c, w3, w4, l, r, pp, f4_bits(cb));
                     if (m.e_frame())
                         u = rs_frame(u, *reinterpret_cast<const float4*>(rs_smem + t.fx + 4 * ec),
-                                     rs_smem[t.fz + er], m.e_xm(), kc.z);
+                                     rs_smem[t.fz + m.er()], m.e_xm(), kc.z);
                     if (m.e_spec())
-                        u = rs_special(u, nxt, er, ec, par, nb, m.e_xm(), rec_out, inject);
-                    if (m.e_write()) st_f4(np, u);
+                        u = rs_special(u, nxt, m.er(), ec, par, m3 == 0 ? 2 : m3 - 1, m.e_xm(),
+                                       pitch, !fwd && k < 2 * nt - 1);
                     float v[4];
                     f4_get(u, v);
-                    uint4* out = s.xbuf + (tag & 1u) * t.half;
                     if (m.ox >= 0)
                         rs_send(out + m.ox, ec == 0 ? v[0] : v[2], ec == 0 ? v[1] : v[3], tag);
                     if (m.oz >= 0) {
                         rs_send(out + m.oz, v[0], v[1], tag);
                         rs_send(out + m.oz + 1, v[2], v[3], tag);
                     }
+                    if (m.e_write()) st_f4(np, u);
+                }
+                RsFused fu{nullptr, nullptr, false};
+                if (on) {
+                    if (s.snaps) {
+                        float* sn = s.snaps + (size_t)(ks - s.slot0) * s.plane;
+                        if (fwd) fu.snap_out = sn;
+                        else if (s.image && ks < s.n_snaps) fu.snap_in = sn;
+                    }
+                    fu.acc = fwd ? s.illum != nullptr : fu.snap_in != nullptr;
+                }
+                if (e_warp && (fu.acc || fu.snap_out)) {
+                    const int ec = m.ec(), er = m.er();
+                    const F4 c = ld_f4(rs_smem + cur + (er + 2) * pitch + 4 * ec);
+                    if (fu.snap_out && m.e_live())
+                        rs_snap(fu.snap_out + (size_t)(t.z0 + er) * t.ldx + t.x0 + 4 * ec, c);
                     if (fu.acc) {
+                        uint32_t ab[4];
+                        tm_converge();
+                        tm_ld4(m.tm + RS_TM_AE, ab);
+                        float4 fe = make_float4(0.f, 0.f, 0.f, 0.f);
+                        if (fu.snap_in && m.e_live())
+                            fe = *reinterpret_cast<const float4*>(
+                                fu.snap_in + (size_t)(t.z0 + er) * t.ldx + t.x0 + 4 * ec);
+                        tm_wait_ld(ab);
                         const f32x2 dt = pk(s.img_dt, s.img_dt);
-                        const F4 acc = fu.snap_in ? rs_image(f4_bits(ab), c, f, dt, kc.z)
+                        const F4 acc = fu.snap_in ? rs_image(f4_bits(ab), c, fe, dt, kc.z)
                                                   : rs_illum(f4_bits(ab), c, kc.z);
                         uint32_t o[4];
                         bits_f4(acc, o);
                         tm_converge();
                         tm_st4(m.tm + RS_TM_AE, o);
+                        tm_wait_st();
                     }
-                    if (fu.snap_out && m.e_live()) rs_snap(fu.snap_out + eo, c);
                 }
                 // ---- phase I
                 tm_converge();
                 if (i_warp) {
-                    if (fused)
-                        rs_inner<true>(m, kc, cur, nxt, t.R, fu, pk(s.img_dt, s.img_dt));
+                    if (fu.acc || fu.snap_out)
+                        rs_inner<true>(m, kc, pitch, cur, nxt, t.R, fu, pk(s.img_dt, s.img_dt));
                     else
-                        rs_inner<false>(m, kc, cur, nxt, t.R, fu, 0);
+                        rs_inner<false>(m, kc, pitch, cur, nxt, t.R, fu, 0);
                     for (unsigned b = m.spec(); b; b &= b - 1) {
                         const int r = m.r0() + __ffs(b) - 1, c = m.c();
-                        float* o = rs_smem + nxt + (r + 2) * t.pitch + 4 * c;
-                        st_f4(o, rs_special(ld_f4(o), nxt, r, c, par, nb, m.i_xm(), rec_out,
-                                            inject));
+                        float* o = rs_smem + nxt + (r + 2) * pitch + 4 * c;
+                        st_f4(o, rs_special(ld_f4(o), nxt, r, c, par, m3 == 0 ? 2 : m3 - 1,
+                                            m.i_xm(), pitch, !fwd && k < 2 * nt - 1));
                     }
-                } else if (fu.acc) {
-                    tm_wait_st();
+                    __syncwarp();
                 }
+                bad = !rs_collect<2>(s.xbuf + t.in + (tag & 1u) * t.half, tag, nxt, par ^ 1,
+                                     t.next + par, s.err);
             } else {
-                // ---- halo warp: the next step's injection, the next snapshot, the edges
+                // ---- halo warp: the last step's samples, the next step's injection, the
+                // next snapshot, the edges
+                if (k > ka && t.rec_row >= 0 && rec_row_out(k - 1))
+                    rs_sample(rec_row_out(k - 1), cur, par ^ 1);
                 const bool more = k + 1 < kb;
                 const float* d = more ? data_row(k + 1) : nullptr;
                 if (t.rec_row >= 0)  // (before the packets: those are still on their way)
@@ -879,10 +916,14 @@ static __global__ void __launch_bounds__(RS_T, 1)
                                                  (size_t)(t.z0 + r) * t.ldx + t.x0,
                                              (uint32_t)t.pitch * 4u);
                 }
-                bad = !rs_collect(s.xbuf + t.in + (tag & 1u) * t.half, tag, nxt, par ^ 1, s.err);
+                if (lane == 0) reinterpret_cast<int*>(rs_smem)[t.next + (par ^ 1)] = 0;
+                __syncwarp();
+                bad = !rs_collect<RS_FLIGHT>(s.xbuf + t.in + (tag & 1u) * t.half, tag, nxt,
+                                             par ^ 1, t.next + par, s.err);
                 if (lane == 0) rs_smem[t.injs + (par ^ 1)] = ns;
             }
             m3 = m3 == 2 ? 0 : m3 + 1;
+            ++tag;
             if (fwd) {
                 if (++rem == s.interval) {
                     rem = 0;
@@ -915,6 +956,8 @@ static __global__ void __launch_bounds__(RS_T, 1)
                 *reinterpret_cast<float4*>(pc + o) = sc[i];
                 *reinterpret_cast<float4*>(pp + o) = sv[i];
             }
+            if (halo && t.rec_row >= 0 && rec_row_out(kb - 1))
+                rs_sample(rec_row_out(kb - 1), RS_PLANE0 + (par ? dpl : 0), par ^ 1);
             if (t.rec_row >= 0 && tid < 4) {
                 const int ix = tid < 2 ? tid : t.nx - 4 + tid;
                 if (ix >= t.x0 && ix < t.x0 + t.pitch)

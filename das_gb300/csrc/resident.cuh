@@ -15,7 +15,7 @@ constexpr int RS_MAXR = 15;         // rows of one phase-I thread: its tensor-me
 constexpr int RS_SMEM = 227 * 1024; // always the whole SM: no second CTA, which could wait
                                     // for tensor memory while its neighbours wait for it
 constexpr int RS_POLLS = 1 << 21;    // looks at a missing packet before giving up (about 1 s)
-constexpr int RS_FLIGHT = 11;       // packets a halo lane has in flight
+constexpr int RS_FLIGHT = 8;       // packets a lane of the halo warp has in flight
 
 // One shot (or one pass of it) as the resident kernel runs it.  Phase step k is forward
 // step k for k < nt, else backward step 2*nt-1-k.
@@ -61,7 +61,7 @@ constexpr int RS_TILE_FLOATS = 64, RS_SHOT_FLOATS = 96;  // the tile's and the s
 __host__ __device__ inline size_t rs_smem_floats(int nrows, int ncol)
 {
     const size_t pitch = 4 * (size_t)ncol;
-    return RS_TILE_FLOATS + RS_SHOT_FLOATS + 2 * (nrows + 4) * pitch + 8 * (size_t)nrows + 4 * pitch + (nrows + 3) / 4 * 4 + 16;
+    return RS_TILE_FLOATS + RS_SHOT_FLOATS + 2 * (nrows + 4) * pitch + 8 * (size_t)nrows + 4 * pitch + (nrows + 3) / 4 * 4 + 24;
 }
 
 // Phase I of a tile: columns 1..ncol-2 by rows 2..nrows-3 in segments of R rows.
@@ -95,7 +95,10 @@ inline std::vector<RsPlan> rs_plans(int nx, int nz, int max_ctas)
             if (R > RS_MAXR) continue;
             const double warps = std::max(1.0, nci * nseg / 32.0);
             const double inner = R ? (R + 1.5) * std::max(warps / 4 * 75.0, 150.0) : 0.0;
-            const double cost = 600.0 + ne / 128.0 * 110.0 + inner + std::max(0.0, 1200.0 - inner);
+            // the packets: their way, then a round trip for every 20 groups
+            const double groups = (2 * nrows + 8 * ncol) / 32.0;
+            const double exchange = 1700.0 + std::max(0.0, groups - 8.0) / 20.0 * 1000.0;
+            const double cost = 500.0 + ne / 128.0 * 110.0 + std::max(inner + 250.0, exchange);
             RsPlan& b = best[gx * gz];
             if (b.ok() && b.cost <= cost) continue;
             b.gx = gx;
