@@ -493,6 +493,7 @@ struct FwdOpts {
     float* snaps = nullptr;      // snapshot slots, slot index = it/interval - slot0
     int slot0 = 0;
     bool illum = false;
+    bool lap = false;            // the snapshots hold the Laplacian of the field (resident form)
     float* ckpt = nullptr;       // save state every ckpt_every steps (3 planes per checkpoint)
     int ckpt_every = 0;
 };
@@ -537,6 +538,7 @@ int run_forward_steps(w2d_engine* e, int slot, const FwdOpts& o, int it0, int it
             r.snaps = o.snaps;
             r.slot0 = o.slot0;
             r.illum = o.illum ? e->illum.p : nullptr;
+            r.lap = o.lap;
             r.wavelet = e->cur_w;
             r.rec_out = o.rec_out;
             r.dt2_inj = dt2inj_f;
@@ -1607,10 +1609,44 @@ __global__ void fwi_chain_kernel(float* grad_v, const float* grad_c, const float
     }
 }
 
+// The gradient passes in the resident form (RsShot::adjoint): q[nt] = c s r[nt-1] at the
+// receivers (one per column), and dJ/dv = 2/v sum q L P (dc/dv = 2 c/v; zero where v is).
+__global__ void fwi_first_kernel(float* q, AcGeom g, const float* c, const float* resid)
+{
+    const int ix = blockIdx.x * blockDim.x + threadIdx.x;
+    if (ix >= g.nx) return;
+    const int k = g.rec_ptr[ix], iz = g.shot[2];
+    if (g.rec_ptr[ix + 1] == k) return;
+    const int d = sponge_dist(ix, iz, g.nx, g.nz, g.n_sponge, g.free_surface);
+    const float sp = g.sponge_lut && d > 0 ? g.sponge_lut[d] : 1.0f;
+    const size_t o = (size_t)iz * g.ldx + ix;
+    q[o] = fmul(resid[g.rec_list[k]], fmul(c[o], sp));
+}
+
+__global__ void fwi_chain_q_kernel(float* grad_v, const float* sum, const float* vel_p, int nx,
+                                   int nz, int ldx)
+{
+    const size_t n = (size_t)nx * nz;
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
+         i += (size_t)gridDim.x * blockDim.x) {
+        const int iz = (int)(i / nx), ix = (int)(i % nx);
+        const size_t o = (size_t)iz * ldx + ix;
+        const float v = vel_p[o];
+        grad_v[i] = v != 0.0f ? __fdiv_rn(2.0f * sum[o], v) : 0.0f;
+    }
+}
+
 bool written_cell(const w2d_engine* e, int iz, int ix)
 {
     const bool interior = iz >= 2 && iz < e->nz - 2 && ix >= 2 && ix < e->nx - 2;
     return interior || (e->fs && iz >= 0 && iz < 2 && ix >= 0 && ix < e->nx);
+}
+
+// Whether the gradient runs in the resident form: when the passes do (receivers on interior
+// rows then sit on interior cells), and the per-cell adjoint was not asked for.
+bool fwi_resident(const w2d_engine* e, int n_rec)
+{
+    return !e->adj_cells && resident(e, n_rec, true);
 }
 
 }  // namespace
@@ -1618,6 +1654,7 @@ bool written_cell(const w2d_engine* e, int iz, int ix)
 struct w2d_fwi_state {
     int nt = 0, n_rec = 0, seg = 0, n_seg = 0;
     bool stored = false;  // one segment of every forward state, written by the forward pass
+    bool lap = false;     // ... as its Laplacian, for the gradient in the resident form
     DevBuf<float> vel_p, grad_c, zero, segbuf;
     std::vector<CUtensorMap> seg_maps;
     CUtensorMap map_c_halo, map_zero;
@@ -1672,7 +1709,9 @@ int w2d_fwi_forward(w2d_engine* e, const float* vel_dev, const float* wavelet, i
     o.n_rec = n_rec;
     o.rec_out = e->rec_out.p;
     f->stored = f->seg >= nt;
+    f->lap = f->stored && fwi_resident(e, n_rec);
     if (f->stored) {
+        o.lap = f->lap;
         // every forward state kept as it is computed: the gradient recomputes nothing
         o.snaps = f->segbuf.p;
         o.interval = 1;
@@ -1717,6 +1756,53 @@ int w2d_fwi_gradient(w2d_engine* e, const float* resid_dev, float* grad_dev)
                                  cudaMemcpyDeviceToDevice, e->stream));
     if ((rc = zero_pass(e, 1))) return rc;
     W2D_CUDA_TRY(cudaMemsetAsync(f->grad_c.p, 0, plane_b, e->stream));
+    if (f->stored ? f->lap : fwi_resident(e, n_rec)) {
+        // q[nt] from the last residuals; then, segment by segment, L P recomputed and the
+        // adjoint imaged with it
+        e->last_launches = 0;
+        e->last_recompute = 0;
+        const AcGeom g = geom(e);
+        fwi_first_kernel<<<(e->nx + 255) / 256, 256, 0, e->stream>>>(
+            e->wave(4), g, e->v2dt2.p, e->data.p + (size_t)(nt - 1) * n_rec);
+        W2D_CUDA_TRY(cudaGetLastError());
+        const float dt2inj = (float)(e->dt_d * e->dt_d);
+        for (int sgi = f->n_seg - 1; sgi >= 0; --sgi) {
+            const int a = sgi * seg, b = std::min(nt, a + seg);
+            if (!f->stored) {
+                const float* c = e->ckpt.p + (size_t)sgi * 3 * e->plane;
+                for (int i = 0; i < 3; ++i)
+                    W2D_CUDA_TRY(cudaMemcpyAsync(e->wave((a + i) % 3), c + i * e->plane, plane_b,
+                                                 cudaMemcpyDeviceToDevice, e->stream));
+                FwdOpts r;
+                r.nt = nt;
+                r.interval = 1;
+                r.snaps = f->segbuf.p;
+                r.slot0 = a;
+                r.lap = true;
+                if ((rc = run_forward_steps(e, 0, r, a, b, 0.0, dt2inj))) return rc;
+                e->last_recompute += b - a;
+            }
+            RsShot s = rs_shot(e);
+            s.src_ix = -1;
+            s.adjoint = 1;
+            s.nt = nt;
+            s.interval = 1;
+            s.k0 = 2 * nt - b;
+            s.k1 = 2 * nt - a;
+            s.vel[1] = e->v2dt2.p;
+            s.snaps = f->segbuf.p;
+            s.slot0 = a;
+            s.n_snaps = b;
+            s.image = f->grad_c.p;
+            s.data = e->data.p;
+            s.img_dt = 1.0f;
+            if ((rc = rs_run(e, s))) return rc;
+        }
+        fwi_chain_q_kernel<<<grid_for((size_t)e->nx * e->nz), 256, 0, e->stream>>>(
+            grad_dev, f->grad_c.p, f->vel_p.p, e->nx, e->nz, e->ldx);
+        W2D_CUDA_TRY(cudaGetLastError());
+        return check_err(e);
+    }
     const int hz = e->tile.tz() + 4;
     if ((rc = make_tensor_map_2d(&f->map_c_halo, e->v2dt2.p, e->nx, e->nz, e->ldx, AC_SW, hz)) ||
         (rc = make_tensor_map_2d(&f->map_zero, f->zero.p, e->nx, e->nz, e->ldx, AC_SW, hz)))

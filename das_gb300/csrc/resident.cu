@@ -29,7 +29,8 @@
 //     arithmetic; from the adjacent lanes, by shuffles and selects, they cost ten more
 //     instructions of a hundred.)
 //   * The halo warp collects the neighbours' edges meanwhile into the halo of p_next,
-//     stages the next step's injection values, and prefetches the next snapshot into L2.
+//     samples the receivers of the last step, stages the next step's injection values, and
+//     prefetches the next snapshot into L2.
 // One barrier ends the step.
 //
 // Exchange: 16-byte packets {value, tag, value, tag} in global memory, tag = step
@@ -110,6 +111,11 @@ __device__ __forceinline__ void f4_get(const F4& v, float u[4])
 {
     upk(v.a, u[0], u[1]);
     upk(v.b, u[2], u[3]);
+}
+__device__ __forceinline__ F4 f4_neg(const F4& v)
+{
+    const f32x2 sign = 0x8000000080000000ull;
+    return F4{v.a ^ sign, v.b ^ sign};
 }
 __device__ __forceinline__ F4 f4_of(const float u[4]) { return F4{pk(u[0], u[1]), pk(u[2], u[3])}; }
 
@@ -193,7 +199,7 @@ struct RsConst {
 };
 __device__ __forceinline__ F4 rs_stencil(const RsConst& k, const F4& w0, const F4& w1, const F4& c,
                                          const F4& w3, const F4& w4, f32x2 l, f32x2 r,
-                                         const F4& pp, const F4& v)
+                                         const F4& pp, const F4& v, F4& lap)
 {
     float cx, cy, cz, cw, l2, l1, r1, r2;
     upk(l, l2, l1);
@@ -212,9 +218,11 @@ __device__ __forceinline__ F4 rs_stencil(const RsConst& k, const F4& w0, const F
     const f32x2 zb = mul(add2(add2(mul(k.k2, add2(w0.b, w4.b)), mul(k.k1, add2(w1.b, w3.b))),
                               kcb), k.dz2);
     // v*lap + (2c - pp), the second term as -(pp - 2c): 2c is exact, so one rounding
+    lap.a = add2(xa, za);
+    lap.b = add2(xb, zb);
     F4 u;
-    u.a = sub2(mul(v.a, add2(xa, za)), fma2(c.a, k.m2, pp.a));
-    u.b = sub2(mul(v.b, add2(xb, zb)), fma2(c.b, k.m2, pp.b));
+    u.a = sub2(mul(v.a, lap.a), fma2(c.a, k.m2, pp.a));
+    u.b = sub2(mul(v.b, lap.b), fma2(c.b, k.m2, pp.b));
     return u;
 }
 
@@ -394,9 +402,11 @@ static_assert(RS_MAXR <= 15, "rows with a rule: 15 bits");
 
 // What this step does beside the stencil.
 struct RsFused {
-    float* snap_out;         // forward: copy of p_curr
+    float* snap_out;         // forward: copy of p_curr, or (lap) its Laplacian
     const float* snap_in;    // backward: the forward snapshot to image with
     bool acc;                // illumination or image
+    bool lap;
+    bool fold;               // adjoint under a free surface: the first row is z = 2
 };
 
 // Phase I of one step: rows of one unit column.  FUSED: see RsFused.
@@ -445,7 +455,13 @@ __device__ __forceinline__ void rs_inner(const RsMine& m, const RsConst& k, int 
         const F4 w4 = ld_f4(rs_smem + oc + 2 * pitch);
         const F4 pp = ld_f4(rs_smem + oc + dn);
         const f32x2 l = rs_pair(oc - 2), r = rs_pair(oc + 4);
-        F4 u = rs_stencil(k, w0, w1, w2, w3, w4, l, r, pp, v);
+        if (FUSED && i == 0 && fu.fold) {
+            w1 = f4_neg(w2);
+            w0 = f4_neg(w3);
+        }
+        F4 lap;
+        F4 u = rs_stencil(k, w0, w1, w2, w3, w4, l, r, pp, v, lap);
+        if (FUSED && i == 0 && fu.fold) w1 = F4{0, 0};
         if (frame) u = rs_frame(u, fx, rs_smem[ofz + (ok ? i : 0)], m.i_xm(), k.z);
         if (ok) st_f4(rs_smem + oc + dn, u);
         if (FUSED) {
@@ -456,7 +472,7 @@ __device__ __forceinline__ void rs_inner(const RsMine& m, const RsConst& k, int 
                 tm_converge();
                 tm_st4(m.tm + RS_TM_A + 4 * i, o);
             }
-            if (fu.snap_out && ok) rs_snap(fu.snap_out + goff, w2);
+            if (fu.snap_out && ok) rs_snap(fu.snap_out + goff, fu.lap ? lap : w2);
             f = f1;
             f1 = f2;
             goff += t.ldx;
@@ -585,7 +601,7 @@ static __global__ void __launch_bounds__(RS_T, 1)
                              s.src_iz < w.z0 + nrows;
         w.src_row = has_src ? s.src_iz - w.z0 : -1;
         w.src_x = has_src ? s.src_ix - w.x0 : -1;
-        w.mirror = s.fs && w.z0 <= 2 && w.z0 + nrows > 2 ? 2 - w.z0 : -1;
+        w.mirror = s.fs && !s.adjoint && w.z0 == 0 ? 2 : -1;  // (a tile has 4 rows or more)
         // packets of one slot of one tile; a tile's slot holds the packets from its left,
         // right, upper and lower neighbour, as many as it has
         const int half = 2 * s.maxr + 8 * s.maxc;
@@ -706,6 +722,7 @@ static __global__ void __launch_bounds__(RS_T, 1)
     bool bad = false;
     unsigned tag = s.tag0 + 1u;
     const int pitch = t.pitch, dpl = t.plane[1] - t.plane[0];
+    const bool adj_top = s.adjoint && s.fs && t.z0 == 0;
 
     for (int ka = s.k0; ka < s.k1 && !bad;) {
         // the steps of one pass
@@ -727,6 +744,12 @@ static __global__ void __launch_bounds__(RS_T, 1)
         };
         auto rec_row_out = [&](int k) {
             return fwd && s.rec_out ? s.rec_out + (size_t)k * s.n_rec : nullptr;
+        };
+        // what the receiver row's data are scaled by: dt^2, or (adjoint) c s of the cell
+        auto inj_factor = [&](int c) {
+            if (!s.adjoint) return s.dt2_inj;
+            const float v = s.vel[1][(size_t)s.rec_iz * t.ldx + t.x0 + c];
+            return fmul(v, fminf(rs_smem[t.fx + c], rs_smem[t.fz + t.rec_row]));
         };
         auto rec_of = [&](int c) { return __float_as_int(rs_smem[t.rk + c]); };
         // ---- the state into the SM
@@ -785,7 +808,7 @@ static __global__ void __launch_bounds__(RS_T, 1)
                 const float* d = data_row(ka);
                 for (int c = lane; c < t.pitch; c += 32) {
                     const int r = rec_of(c);
-                    rs_smem[t.inj + c] = d && r >= 0 ? fmul(d[r], s.dt2_inj) : -0.0f;
+                    rs_smem[t.inj + c] = d && r >= 0 ? fmul(d[r], inj_factor(c)) : -0.0f;
                 }
                 if (lane == 0) rs_smem[t.injs] = src_value(ka);
             }
@@ -812,14 +835,19 @@ static __global__ void __launch_bounds__(RS_T, 1)
                     const F4 c = ld_f4(rs_smem + oc);
                     const f32x2 l = rs_pair(ec > 0 ? oc - 2 : m.hx(par)),
                                 r = rs_pair(m.last_col() ? m.hx(par) : oc + 4);
-                    const F4 w0 = ld_f4(rs_smem + oc - 2 * pitch), w1 = ld_f4(rs_smem + oc - pitch),
-                             w3 = ld_f4(rs_smem + oc + pitch),
+                    F4 w0 = ld_f4(rs_smem + oc - 2 * pitch), w1 = ld_f4(rs_smem + oc - pitch);
+                    const F4 w3 = ld_f4(rs_smem + oc + pitch),
                              w4 = ld_f4(rs_smem + oc + 2 * pitch);
+                    if (adj_top && m.er() == 2) {
+                        w1 = f4_neg(c);
+                        w0 = f4_neg(w3);
+                    }
                     float* np = rs_smem + oc + nxt - cur;
                     const F4 pp = ld_f4(np);
                     uint4* out = s.xbuf + (tag & 1u) * t.half;
                     tm_wait_ld(cb);
-                    F4 u = rs_stencil(kc, w0, w1, c, w3, w4, l, r, pp, f4_bits(cb));
+                    F4 lap;
+                    F4 u = rs_stencil(kc, w0, w1, c, w3, w4, l, r, pp, f4_bits(cb), lap);
                     if (m.e_frame())
                         u = rs_frame(u, *reinterpret_cast<const float4*>(rs_smem + t.fx + 4 * ec),
                                      rs_smem[t.fz + m.er()], m.e_xm(), kc.z);
@@ -835,9 +863,13 @@ static __global__ void __launch_bounds__(RS_T, 1)
                         rs_send(out + m.oz + 1, v[2], v[3], tag);
                     }
                     if (m.e_write()) st_f4(np, u);
+                    if (on && fwd && s.lap && m.e_live())
+                        rs_snap(s.snaps + (size_t)(ks - s.slot0) * s.plane +
+                                    (size_t)(t.z0 + m.er()) * t.ldx + t.x0 + 4 * ec, lap);
                 }
-                RsFused fu{nullptr, nullptr, false};
+                RsFused fu{nullptr, nullptr, false, false, adj_top && m.r0() == 2};
                 if (on) {
+                    fu.lap = fwd && s.lap;
                     if (s.snaps) {
                         float* sn = s.snaps + (size_t)(ks - s.slot0) * s.plane;
                         if (fwd) fu.snap_out = sn;
@@ -848,7 +880,7 @@ static __global__ void __launch_bounds__(RS_T, 1)
                 if (e_warp && (fu.acc || fu.snap_out)) {
                     const int ec = m.ec(), er = m.er();
                     const F4 c = ld_f4(rs_smem + cur + (er + 2) * pitch + 4 * ec);
-                    if (fu.snap_out && m.e_live())
+                    if (fu.snap_out && !fu.lap && m.e_live())
                         rs_snap(fu.snap_out + (size_t)(t.z0 + er) * t.ldx + t.x0 + 4 * ec, c);
                     if (fu.acc) {
                         uint32_t ab[4];
@@ -899,7 +931,7 @@ static __global__ void __launch_bounds__(RS_T, 1)
 #pragma unroll
                         for (int j = 0; j < 8; ++j) {
                             const int c = c0 + 32 * j, r = d && c < t.pitch ? rec_of(c) : -1;
-                            v[j] = r >= 0 ? fmul(d[r], s.dt2_inj) : -0.0f;
+                            v[j] = r >= 0 ? fmul(d[r], inj_factor(c)) : -0.0f;
                         }
 #pragma unroll
                         for (int j = 0; j < 8; ++j)

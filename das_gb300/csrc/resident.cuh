@@ -32,6 +32,13 @@ struct RsShot {
     const float* vel[2];       // v^2 dt^2 of the forward and the backward pass
     float* snaps;              // forward: written when not null; backward: read when imaging
     int slot0, n_snaps;        // first snapshot held; snapshots that exist (backward)
+    // The velocity gradient.  With q = c a, c = v^2 dt^2, the adjoint of the step
+    // (adjoint_kernels.cuh) is the step itself: q[n] = s (2 q[n+1] - q[n+2] + c (L q[n+1] +
+    // r[n-1])), and dJ/dc = (1/c) sum_n q[n+1] L P[n].  So (lap) the forward pass keeps
+    // L P[n], which it computes anyway, in place of P[n], and (adjoint) the backward pass
+    // images with it, its receivers' injection times c s, its free surface the transpose
+    // of the forward one: row 2 reads -q[2] and -q[3] for rows 1 and 0, which stay zero.
+    int lap, adjoint;
     size_t plane;
     float* illum;              // forward: accumulated when not null
     float* image;              // backward: accumulated when not null
