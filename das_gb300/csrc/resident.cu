@@ -29,8 +29,7 @@
 //     arithmetic; from the adjacent lanes, by shuffles and selects, they cost ten more
 //     instructions of a hundred.)
 //   * The halo warp collects the neighbours' edges meanwhile into the halo of p_next,
-//     samples the receivers of the last step, stages the next step's injection values, and
-//     prefetches the next snapshot into L2.
+//     samples the receivers of the last step, and prefetches the next snapshot into L2.
 // One barrier ends the step.
 //
 // Exchange: 16-byte packets {value, tag, value, tag} in global memory, tag = step
@@ -760,6 +759,7 @@ static __global__ void __launch_bounds__(RS_T, 1)
             const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
             float4 *d0 = reinterpret_cast<float4*>(rs_smem + t.plane[0]),
                    *d1 = reinterpret_cast<float4*>(rs_smem + t.plane[1]);
+#pragma unroll 4
             for (int i = tid; i < (nrows + 4) * ncol; i += RS_T) {
                 const int r = i / ncol - 2, c = i - (r + 2) * ncol, iz = t.z0 + r;
                 const size_t o = (size_t)iz * ldx + t.x0 + 4 * c;
@@ -788,20 +788,35 @@ static __global__ void __launch_bounds__(RS_T, 1)
             if (!halo) {  // tensor memory: every lane of a warp takes part
                 const float* vel = s.vel[fwd ? 0 : 1];
                 const float* accg = fwd ? s.illum : s.image;
-                auto put = [&](const float* p, bool ok, size_t o, int word) {
-                    uint32_t r[4] = {0, 0, 0, 0};
-                    if (p && ok) bits_of(*reinterpret_cast<const float4*>(p + o), r);
+                auto get = [&](const float* p, bool ok, size_t o) {
+                    return p && ok ? *reinterpret_cast<const float4*>(p + o)
+                                   : make_float4(0.f, 0.f, 0.f, 0.f);
+                };
+                auto put = [&](const float4& v, int word) {
+                    uint32_t r[4];
+                    bits_of(v, r);
                     tm_converge();
                     tm_st4(m.tm + word, r);
                 };
                 const size_t eo = (size_t)(t.z0 + m.er()) * ldx + t.x0 + 4 * m.ec();
-                put(vel, m.e_live(), eo, RS_TM_CE);
-                put(accg, m.e_live(), eo, RS_TM_AE);
+                const float4 ev = get(vel, m.e_live(), eo), ea = get(accg, m.e_live(), eo);
+                put(ev, RS_TM_CE);
+                put(ea, RS_TM_AE);
                 if (i_warp)
-                    for (int i = 0; i < t.R; ++i) {
-                        const size_t o = (size_t)(t.z0 + m.r0() + i) * ldx + t.x0 + 4 * m.c();
-                        put(vel, i < m.n(), o, RS_TM_C + 4 * i);
-                        put(accg, i < m.n(), o, RS_TM_A + 4 * i);
+                    for (int i0 = 0; i0 < t.R; i0 += 5) {  // five rows under way at a time
+                        float4 v[5], a[5];
+                        const size_t o = (size_t)(t.z0 + m.r0() + i0) * ldx + t.x0 + 4 * m.c();
+#pragma unroll
+                        for (int j = 0; j < 5; ++j) {
+                            v[j] = get(vel, i0 + j < m.n(), o + (size_t)j * ldx);
+                            a[j] = get(accg, i0 + j < m.n(), o + (size_t)j * ldx);
+                        }
+#pragma unroll
+                        for (int j = 0; j < 5; ++j)
+                            if (i0 + j < RS_MAXR) {
+                                put(v[j], RS_TM_C + 4 * (i0 + j));
+                                put(a[j], RS_TM_A + 4 * (i0 + j));
+                            }
                     }
                 tm_wait_st();
             } else {
@@ -826,6 +841,18 @@ static __global__ void __launch_bounds__(RS_T, 1)
             const int cur = RS_PLANE0 + (par ? dpl : 0), nxt = RS_PLANE0 + (par ? 0 : dpl);
             const bool on = rem == 0;  // a step with a snapshot
             if (!halo) {
+                // the next step's injection, a column a thread: on its way from here, staged at
+                // the end of the step
+                float nd = -0.0f, nf = 1.0f;
+                const bool stage = !fwd && t.rec_row >= 0 && tid < pitch;
+                if (stage && k + 1 < kb) {
+                    const float* d = data_row(k + 1);
+                    const int r = rec_of(tid);
+                    if (d && r >= 0) {
+                        nd = d[r];
+                        nf = inj_factor(tid);
+                    }
+                }
                 // ---- phase E
                 if (e_warp) {
                     const int ec = m.ec(), oc = cur + (m.er() + 2) * pitch + 4 * ec;
@@ -916,6 +943,8 @@ static __global__ void __launch_bounds__(RS_T, 1)
                     }
                     __syncwarp();
                 }
+                if (stage) rs_smem[t.inj + (par ^ 1) * pitch + tid] = fmul(nd, nf);
+                __syncwarp();
                 bad = !rs_collect<2>(s.xbuf + t.in + (tag & 1u) * t.half, tag, nxt, par ^ 1,
                                      t.next + par, s.err);
             } else {
@@ -924,19 +953,12 @@ static __global__ void __launch_bounds__(RS_T, 1)
                 if (k > ka && t.rec_row >= 0 && rec_row_out(k - 1))
                     rs_sample(rec_row_out(k - 1), cur, par ^ 1);
                 const bool more = k + 1 < kb;
-                const float* d = more ? data_row(k + 1) : nullptr;
-                if (t.rec_row >= 0)  // (before the packets: those are still on their way)
-                    for (int c0 = lane; c0 < t.pitch; c0 += 256) {
-                        float v[8];
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) {
-                            const int c = c0 + 32 * j, r = d && c < t.pitch ? rec_of(c) : -1;
-                            v[j] = r >= 0 ? fmul(d[r], inj_factor(c)) : -0.0f;
-                        }
-#pragma unroll
-                        for (int j = 0; j < 8; ++j)
-                            if (c0 + 32 * j < t.pitch)
-                                rs_smem[t.inj + (par ^ 1) * t.pitch + c0 + 32 * j] = v[j];
+                if (t.rec_row >= 0)  // columns past the compute threads'
+                    for (int c = RS_CT + lane; c < pitch; c += 32) {
+                        const float* d = more ? data_row(k + 1) : nullptr;
+                        const int r = rec_of(c);
+                        rs_smem[t.inj + (par ^ 1) * pitch + c] =
+                            d && r >= 0 ? fmul(d[r], inj_factor(c)) : -0.0f;
                     }
                 float ns = -0.0f;
                 if (lane == 0 && more) ns = src_value(k + 1);
@@ -982,6 +1004,7 @@ static __global__ void __launch_bounds__(RS_T, 1)
                 reinterpret_cast<const float4*>(rs_smem + t.plane[par] + 2 * t.pitch);
             const float4* sv =
                 reinterpret_cast<const float4*>(rs_smem + t.plane[par ^ 1] + 2 * t.pitch);
+#pragma unroll 4
             for (int i = tid; i < nrows * ncol; i += RS_T) {
                 const int r = i / ncol, c = i - r * ncol;
                 const size_t o = (size_t)(t.z0 + r) * ldx + t.x0 + 4 * c;

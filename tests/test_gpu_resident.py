@@ -110,3 +110,45 @@ def test_batch_waves_equal_steps():
                 np.testing.assert_array_equal(r[1], ill)
             s.close()
     eng.close()
+
+
+@pytest.mark.parametrize("nz,nx,fs,n_sponge,riz,rstep,nt,seg", [
+    (8, 9, True, 2, 2, 1, 40, 0),        # one tile; the fold's rows 2 and 3 at a tile's edge
+    (9, 37, True, 3, 3, 1, 30, 7),
+    (61, 261, True, 10, 2, 2, 90, 0),
+    (60, 262, False, 10, 13, 1, 90, 90),  # every state stored
+    (150, 403, True, 40, 2, 3, 200, 0),
+    (700, 1990, False, 30, 36, 1, 60, 0),
+])
+def test_resident_gradient_equals_adjoint_kernels(nz, nx, fs, n_sponge, riz, rstep, nt, seg):
+    """The velocity gradient with the adjoint on chip against the adjoint kernels: traces
+    equal, the gradient to float32 rounding (a sum of nt products, each with a few
+    roundings of 6e-8: 1e-5 holds with room, as between the two adjoint kernels)."""
+    import torch
+    from das_gb300.autograd import model_traces
+    from das_gb300.wave_solver import WaveSolver2D
+    rng = np.random.default_rng(nz + nx)
+    v = (2000.0 + 300.0 * rng.random((nz, nx))).astype(np.float32)
+    v[nz // 2, nx // 2] = 0.0  # no gradient where the velocity is zero
+    w = rng.standard_normal(nt).astype(np.float32)
+    rix = np.arange(2, nx - 2, rstep)
+    r = torch.tensor(rng.standard_normal((nt, len(rix))).astype(np.float32), device="cuda")
+    out = []
+    for pdl in (True, False):
+        s = WaveSolver2D(nx, nz, 5.0, 5.0, 5e-4, n_sponge=n_sponge, free_surface_top=fs)
+        s.set_launch("grid", pdl)
+        if seg:
+            s.set_checkpoint_segment(seg)
+        g = []
+        for _ in range(2):
+            vt = torch.tensor(v, device="cuda", requires_grad=True)
+            d = model_traces(vt, s, w, nx // 3, min(max(riz, 2), nz - 3), rix, riz)
+            d.backward(r)
+            g.append((d.detach().cpu().numpy(), vt.grad.cpu().numpy()))
+        np.testing.assert_array_equal(g[0][1], g[1][1])
+        out.append(g[0])
+        s.close()
+    np.testing.assert_array_equal(out[0][0], out[1][0])
+    a, b = (x[1].astype(np.float64) for x in out)
+    assert np.isfinite(a).all() and a[nz // 2, nx // 2] == 0.0
+    assert np.linalg.norm(a - b) <= 1e-5 * np.linalg.norm(b)
