@@ -69,9 +69,9 @@ struct ElAdjRecv {
 };
 
 struct ElAdjMaps {
-    CUtensorMap tmp;     // the t / r planes (5 per shot)
-    CUtensorMap f_next;  // u_{n+1}
-    CUtensorMap f_curr;  // u_n
+    CUtensorMap tmp;  // the t / r planes (5 per shot)
+    CUtensorMap fwd;  // forward states: u_n's planes from curr0 on, u_{n+1}'s from next0 on
+    int next0, curr0;
 };
 
 // K2 + K3 of step n
@@ -110,11 +110,11 @@ __global__ void __launch_bounds__(WARPS * 32)
         tma_load_3d(b_txx, &maps.tmp, xs, zs, pb + EL_SXX, bar);
         tma_load_3d(b_txz, &maps.tmp, xs, zs, pb + EL_SXZ, bar);
         tma_load_3d(b_tzz, &maps.tmp, xs, zs, pb + EL_SZZ, bar);
-        tma_load_3d(b_nvx, &maps.f_next, xs, zs, pb + EL_VX, bar);
-        tma_load_3d(b_nvz, &maps.f_next, xs, zs, pb + EL_VZ, bar);
-        tma_load_3d(b_cxx, &maps.f_curr, xs, zs, pb + EL_SXX, bar);
-        tma_load_3d(b_cxz, &maps.f_curr, xs, zs, pb + EL_SXZ, bar);
-        tma_load_3d(b_czz, &maps.f_curr, xs, zs, pb + EL_SZZ, bar);
+        tma_load_3d(b_nvx, &maps.fwd, xs, zs, maps.next0 + pb + EL_VX, bar);
+        tma_load_3d(b_nvz, &maps.fwd, xs, zs, maps.next0 + pb + EL_VZ, bar);
+        tma_load_3d(b_cxx, &maps.fwd, xs, zs, maps.curr0 + pb + EL_SXX, bar);
+        tma_load_3d(b_cxz, &maps.fwd, xs, zs, maps.curr0 + pb + EL_SXZ, bar);
+        tma_load_3d(b_czz, &maps.fwd, xs, zs, maps.curr0 + pb + EL_SZZ, bar);
     }
     const int ixb = x0 + 4 * lane;
     const bool col_ok = ixb < g.ldx;
@@ -483,7 +483,7 @@ inline cudaError_t launch_el_adj_b(const ElAdjMaps& m, const ElGeom& g, const El
     return cudaErrorInvalidValue;
 }
 
-// 3D map over the states (5 planes per shot) of a buffer, with boxes of tile height tz.
+// 3D map over n_shots states (5 planes each) of a buffer, with boxes of tile height tz.
 inline int make_el_adj_map(CUtensorMap* m, const float* base, int nx, int nz, int ldx,
                            size_t plane, int n_shots, int tz = EL_ADJ_WARPS * EL_ADJ_RPW)
 {

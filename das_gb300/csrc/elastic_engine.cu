@@ -59,7 +59,8 @@ struct w2d_elastic {
     bool have_forward = false;
     unsigned* err = nullptr;                // device error word of the step kernels
     CUtensorMap map_state;                  // 3D map over the S x 5 planes of `state`
-    std::vector<CUtensorMap> seg_maps;      // one per slot of `seg`
+    CUtensorMap map_seg;                    // and over all slots of `seg`
+    bool stored = false;                    // `seg` holds every forward state
     int adj_form = 1;                       // 1: TMA-tiled adjoint passes, 0: per-cell kernels
     // every shot of the next batch has the same model: its parameters are stored once and
     // read by every shot (parameter stride 0), so a tile's parameters come from L2 for
@@ -77,7 +78,7 @@ struct w2d_elastic {
     bool chain = false;
     bool last_stress = false;  // ... and that kernel was a stress phase
     CUtensorMap adj_map_tmp;                // the adjoint passes' maps (their own box height)
-    std::vector<CUtensorMap> adj_seg_maps;
+    CUtensorMap adj_map_seg;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     float last_ms = 0.f;
 
@@ -132,17 +133,17 @@ ElStrides estrides(w2d_elastic* e)
     return ElStrides{e->SS(), e->pstride, 4 * e->plane};
 }
 
-// Step n of every shot from the states at src to the states at dst (same pointer:
-// in place), the source term w[n] * dt added to vz at each shot's source first.
-int fwd_step(w2d_elastic* e, const CUtensorMap& msrc, const CUtensorMap& mdst, const float* src,
-             float* dst, int n, float* trace_row = nullptr)
+// Step n of every shot, in place in `state` (slot < 0) or from slot to slot + 1 of `seg`,
+// the source term w[n] * dt added to vz at each shot's source first.
+int fwd_step(w2d_elastic* e, int slot, int n, float* trace_row = nullptr)
 {
     ElMaps m;
-    m.src = msrc;
-    m.dst = mdst;
+    m.src = m.dst = slot < 0 ? e->map_state : e->map_seg;
     ElStep st;
-    st.src = src;
-    st.dst = dst;
+    st.src = slot < 0 ? e->state : e->slot(slot);
+    st.dst = slot < 0 ? e->state : e->slot(slot + 1);
+    st.src_plane0 = slot < 0 ? 0 : 5 * e->S * slot;
+    st.dst_plane0 = slot < 0 ? 0 : 5 * e->S * (slot + 1);
     st.plane = e->plane;
     st.lam = e->P(0, 0);
     st.mu = e->P(0, 1);
@@ -301,6 +302,21 @@ int w2d_elastic_forward_batch(w2d_elastic* e, int n_shots, const float* lam, con
     e->rec_iz = rec_iz;
     plan_segments(nt, &e->seg_len, &e->n_seg);
     const size_t P = e->plane, SS = e->SS();
+    // Every state kept where they all fit an eighth of the free memory (the rest stays for
+    // others): nothing is recomputed (forward and gradient, 4 shots of 363 x 725, 700 steps:
+    // 41.6 -> 31.0 ms; 1024 x 2048, 500 steps: 52.5 -> 41.4).
+    const size_t all = (size_t)(nt + 1) * S * SS;
+    e->stored = false;
+    if ((size_t)(nt + 1) * S * 5 <= 0x7fffffff) {
+        size_t fr = 0, tot = 0;
+        if (all > e->seg_cap) cudaMemGetInfo(&fr, &tot);
+        e->stored = (all <= e->seg_cap || all * 4 <= fr / 8) &&
+                    grow(&e->seg, all, &e->seg_cap) == W2D_OK;
+    }
+    if (e->stored) {
+        e->seg_len = nt;
+        e->n_seg = 1;
+    }
     if ((rc = grow(&e->params, (size_t)S * 4 * P, &e->params_cap)) ||
         (rc = grow(&e->state, (size_t)S * SS, &e->state_cap)) ||
         (rc = grow(&e->adj, (size_t)S * SS, &e->adj_cap)) ||
@@ -312,7 +328,7 @@ int w2d_elastic_forward_batch(w2d_elastic* e, int n_shots, const float* lam, con
         (rc = grow(&e->traces, (size_t)S * nt * n_rec, &e->tr_cap)) ||
         (rc = grow(&e->rec_ptr, (size_t)e->nx + 1, &e->rp_cap)) ||
         (rc = grow(&e->rec_list, (size_t)n_rec, &e->rl_cap)) ||
-        (rc = grow(&e->ckpt, (size_t)e->n_seg * S * SS, &e->ckpt_cap)) ||
+        (!e->stored && (rc = grow(&e->ckpt, (size_t)e->n_seg * S * SS, &e->ckpt_cap))) ||
         (rc = grow(&e->seg, (size_t)(e->seg_len + 1) * S * SS, &e->seg_cap)))
         return rc;
     e->map_fwd_warps = e->fwd_warps;
@@ -322,17 +338,11 @@ int w2d_elastic_forward_batch(w2d_elastic* e, int n_shots, const float* lam, con
     const int ftz = e->fwd_warps * e->fwd_rpw, atz = e->adj_warps * e->adj_rpw;
     if ((rc = make_el_state_map(&e->map_state, e->state, e->nx, e->nz, e->ldx, P, S, ftz)))
         return rc;
-    e->seg_maps.resize(e->seg_len + 1);
-    for (int i = 0; i <= e->seg_len; ++i)
-        if ((rc = make_el_state_map(&e->seg_maps[i], e->slot(i), e->nx, e->nz, e->ldx, P, S, ftz)))
-            return rc;
-    if ((rc = make_el_adj_map(&e->adj_map_tmp, e->tmp, e->nx, e->nz, e->ldx, P, S, atz)))
+    const int n_states = S * (e->seg_len + 1);
+    if ((rc = make_el_state_map(&e->map_seg, e->seg, e->nx, e->nz, e->ldx, P, n_states, ftz)) ||
+        (rc = make_el_adj_map(&e->adj_map_seg, e->seg, e->nx, e->nz, e->ldx, P, n_states, atz)) ||
+        (rc = make_el_adj_map(&e->adj_map_tmp, e->tmp, e->nx, e->nz, e->ldx, P, S, atz)))
         return rc;
-    e->adj_seg_maps.resize(e->seg_len + 1);
-    for (int i = 0; i <= e->seg_len; ++i)
-        if ((rc = make_el_adj_map(&e->adj_seg_maps[i], e->slot(i), e->nx, e->nz, e->ldx, P, S,
-                                  atz)))
-            return rc;
     const size_t hp = (size_t)e->nx * 4, dp = (size_t)e->ldx * 4, np = (size_t)e->nx * e->nz;
     const float* src[4] = {lam, mu, bx, bz};
     const int n_models = e->shared_next ? 1 : S;
@@ -365,18 +375,16 @@ int w2d_elastic_forward_batch(w2d_elastic* e, int n_shots, const float* lam, con
                                      cudaMemcpyHostToDevice, e->st));
         W2D_CUDA_TRY(cudaStreamSynchronize(e->st));  // the host tables die here
     }
-    W2D_CUDA_TRY(cudaMemsetAsync(e->state, 0, (size_t)S * SS * 4, e->st));
+    W2D_CUDA_TRY(cudaMemsetAsync(e->stored ? e->seg : e->state, 0, (size_t)S * SS * 4, e->st));
     W2D_CUDA_TRY(cudaEventRecord(e->e0, e->st));
     e->chain = false;
     for (int n = 0; n < nt; ++n) {
-        if (n % e->seg_len == 0) {
+        if (!e->stored && n % e->seg_len == 0) {
             W2D_CUDA_TRY(cudaMemcpyAsync(e->ckpt + (size_t)(n / e->seg_len) * S * SS, e->state,
                                          (size_t)S * SS * 4, cudaMemcpyDeviceToDevice, e->st));
             e->chain = false;
         }
-        if ((rc = fwd_step(e, e->map_state, e->map_state, e->state, e->state, n,
-                           e->traces + (size_t)n * n_rec)))
-            return rc;
+        if ((rc = fwd_step(e, e->stored ? n : -1, n, e->traces + (size_t)n * n_rec))) return rc;
     }
     e->chain = false;
     W2D_CUDA_TRY(cudaGetLastError());
@@ -439,24 +447,24 @@ int w2d_elastic_gradient_batch(w2d_elastic* e, const float* resid_dev, float* g_
     el_adj_k1<<<grd, blk, 0, e->st>>>(g, prm, sd, a, t);
     for (int sgi = e->n_seg - 1; sgi >= 0; --sgi) {
         const int a0 = sgi * e->seg_len, b0 = std::min(nt, a0 + e->seg_len);
-        // recompute u_a0 .. u_b0 into the segment slots
-        W2D_CUDA_TRY(cudaMemcpyAsync(e->slot(0), e->ckpt + (size_t)sgi * S * SS, (size_t)S * SS * 4,
-                                     cudaMemcpyDeviceToDevice, e->st));
         e->chain = false;
-        // out of place: slot n - a0 keeps u_n (without the w[n] source term)
-        for (int n = a0; n < b0; ++n) {
-            const int i = n - a0;
-            int rc;
-            if ((rc = fwd_step(e, e->seg_maps[i], e->seg_maps[i + 1], e->slot(i), e->slot(i + 1),
-                               n)))
-                return rc;
+        if (!e->stored) {
+            // recompute u_a0 .. u_b0 into the segment slots
+            W2D_CUDA_TRY(cudaMemcpyAsync(e->slot(0), e->ckpt + (size_t)sgi * S * SS,
+                                         (size_t)S * SS * 4, cudaMemcpyDeviceToDevice, e->st));
+            // out of place: slot n - a0 keeps u_n (without the w[n] source term)
+            for (int n = a0; n < b0; ++n) {
+                int rc;
+                if ((rc = fwd_step(e, n - a0, n))) return rc;
+            }
         }
         for (int n = b0 - 1; n >= a0; --n) {
             if (e->adj_form == 1) {
                 ElAdjMaps m;
                 m.tmp = e->adj_map_tmp;
-                m.f_next = e->adj_seg_maps[n + 1 - a0];
-                m.f_curr = e->adj_seg_maps[n - a0];
+                m.fwd = e->adj_map_seg;
+                m.next0 = 5 * S * (n + 1 - a0);
+                m.curr0 = 5 * S * (n - a0);
                 const ElAdjRecv rv{e->traces + (size_t)n * n_rec, tr_stride, e->rec_ptr,
                                    e->rec_list, e->rec_iz};
                 W2D_CUDA_TRY(launch_el_adj_a(m, g, prm, sd, a, r, glam, gmu, gbx, gbz, rv, e->err,

@@ -69,11 +69,12 @@ struct ElStep {
     // the pointwise fields may be staged before the dependency wait: the launch two back
     // wrote them (or nothing running does), see the phases' kernels
     int early = 0;
+    int src_plane0 = 0, dst_plane0 = 0;  // the states' first planes in the maps
 };
 
 struct ElMaps {
-    CUtensorMap src;  // 3D map over the source state's planes
-    CUtensorMap dst;  // 3D map over the destination state's planes
+    CUtensorMap src;  // 3D map over planes with the source state's among them
+    CUtensorMap dst;  // and over the destination state's
 };
 
 constexpr int EL_TX = 128;
@@ -236,9 +237,10 @@ __global__ void __launch_bounds__(WARPS * 32)
     grid_dep_launch();
     if (tid == 0) {
         mbar_expect_tx(bar, 3u * T::BOX * 4u);
-        tma_load_3d(bxx, &maps.src, x0 - EL_HX, z0 - 2, 5 * sh + EL_SXX, bar);
-        tma_load_3d(bxz, &maps.src, x0 - EL_HX, z0 - 2, 5 * sh + EL_SXZ, bar);
-        tma_load_3d(bzz, &maps.src, x0 - EL_HX, z0 - 2, 5 * sh + EL_SZZ, bar);
+        const int pb = s.src_plane0 + 5 * sh;
+        tma_load_3d(bxx, &maps.src, x0 - EL_HX, z0 - 2, pb + EL_SXX, bar);
+        tma_load_3d(bxz, &maps.src, x0 - EL_HX, z0 - 2, pb + EL_SXZ, bar);
+        tma_load_3d(bzz, &maps.src, x0 - EL_HX, z0 - 2, pb + EL_SZZ, bar);
     }
     if (!s.early) el_stage_pointwise<WARPS, RPW>(pt, f, 5, zr0, ixb, lane, warp, g);
     __syncthreads();
@@ -351,8 +353,9 @@ __global__ void __launch_bounds__(WARPS * 32)
     grid_dep_launch();
     if (tid == 0) {
         mbar_expect_tx(bar, 2u * T::BOX * 4u);
-        tma_load_3d(bvx, &maps.dst, x0 - EL_HX, z0 - 2, 5 * sh + EL_VX, bar);
-        tma_load_3d(bvz, &maps.dst, x0 - EL_HX, z0 - 2, 5 * sh + EL_VZ, bar);
+        const int pb = s.dst_plane0 + 5 * sh;
+        tma_load_3d(bvx, &maps.dst, x0 - EL_HX, z0 - 2, pb + EL_VX, bar);
+        tma_load_3d(bvz, &maps.dst, x0 - EL_HX, z0 - 2, pb + EL_VZ, bar);
     }
     if (!s.early) el_stage_pointwise<WARPS, RPW>(pt, f, 6, zr0, ixb, lane, warp, g);
     __syncthreads();
