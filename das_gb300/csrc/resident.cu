@@ -841,18 +841,6 @@ static __global__ void __launch_bounds__(RS_T, 1)
             const int cur = RS_PLANE0 + (par ? dpl : 0), nxt = RS_PLANE0 + (par ? 0 : dpl);
             const bool on = rem == 0;  // a step with a snapshot
             if (!halo) {
-                // the next step's injection, a column a thread: on its way from here, staged at
-                // the end of the step
-                float nd = -0.0f, nf = 1.0f;
-                const bool stage = !fwd && t.rec_row >= 0 && tid < pitch;
-                if (stage && k + 1 < kb) {
-                    const float* d = data_row(k + 1);
-                    const int r = rec_of(tid);
-                    if (d && r >= 0) {
-                        nd = d[r];
-                        nf = inj_factor(tid);
-                    }
-                }
                 // ---- phase E
                 if (e_warp) {
                     const int ec = m.ec(), oc = cur + (m.er() + 2) * pitch + 4 * ec;
@@ -893,6 +881,18 @@ static __global__ void __launch_bounds__(RS_T, 1)
                     if (on && fwd && s.lap && m.e_live())
                         rs_snap(s.snaps + (size_t)(ks - s.slot0) * s.plane +
                                     (size_t)(t.z0 + m.er()) * t.ldx + t.x0 + 4 * ec, lap);
+                }
+                // the next step's injection, a column a thread: on its way from here, staged at
+                // the end of the step
+                float nd = -0.0f, nf = 1.0f;
+                const bool stage = !fwd && t.rec_row >= 0 && tid < pitch;
+                if (stage && k + 1 < kb) {
+                    const float* d = data_row(k + 1);
+                    const int r = rec_of(tid);
+                    if (d && r >= 0) {
+                        nd = d[r];
+                        nf = inj_factor(tid);
+                    }
                 }
                 RsFused fu{nullptr, nullptr, false, false, adj_top && m.r0() == 2};
                 if (on) {

@@ -55,7 +55,7 @@ struct RsShot {
 // ---- host: how a grid is cut -------------------------------------------------------
 struct RsPlan {
     int gx = 0, gz = 0, maxc = 0, maxr = 0;
-    double cost = 0;  // estimated cycles of a step
+    double cost = 0;  // estimated us of a step
     bool ok() const { return gx > 0; }
     int ctas() const { return gx * gz; }
     size_t packets() const { return 2 * (size_t)(2 * maxr + 8 * maxc); }  // of one tile
@@ -86,7 +86,8 @@ __host__ __device__ inline void rs_interior(int nrows, int ncol, int* nci, int* 
 // The cuts of an nx x nz grid: element n is the one into at most n tiles (n = 1 ..
 // max_ctas) with the least estimated step time, none where the grid does not fit the
 // shared memory of n SMs.  What a step costs is its slowest tile, so columns and rows are
-// split evenly and the estimate (in cycles) is that of the largest tile.
+// split evenly and the estimate (in us) is that of the largest tile: a fixed chain, the edge
+// units (columns cost more: their snapshot accesses do not coalesce), the interior.
 inline std::vector<RsPlan> rs_plans(int nx, int nz, int max_ctas)
 {
     std::vector<RsPlan> best(std::max(max_ctas, 0) + 1);
@@ -100,12 +101,9 @@ inline std::vector<RsPlan> rs_plans(int nx, int nz, int max_ctas)
             int nci, nseg, R;
             rs_interior(nrows, ncol, &nci, &nseg, &R);
             if (R > RS_MAXR) continue;
-            const double warps = std::max(1.0, nci * nseg / 32.0);
-            const double inner = R ? (R + 1.5) * std::max(warps / 4 * 75.0, 150.0) : 0.0;
-            // the packets: their way, then a round trip for every 20 groups
-            const double groups = (2 * nrows + 8 * ncol) / 32.0;
-            const double exchange = 1700.0 + std::max(0.0, groups - 8.0) / 20.0 * 1000.0;
-            const double cost = 500.0 + ne / 128.0 * 110.0 + std::max(inner + 250.0, exchange);
+            // fitted to 86 cuts of 7 grids (migrations, every second step imaged): 6 % rms
+            const double warps = (nci * nseg + 31) / 32;
+            const double cost = 1.69 + 0.0087 * nrows + 0.0061 * ncol + 0.019 * R * warps;
             RsPlan& b = best[gx * gz];
             if (b.ok() && b.cost <= cost) continue;
             b.gx = gx;
