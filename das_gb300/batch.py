@@ -235,9 +235,10 @@ class BatchEngine:
         other jobs continue with results unchanged."""
         _lib.check(self._lib.w2d_batch_cancel(self._h, int(slot)))
 
-    def fetch(self, slot: int, nz: int, nx: int) -> Tuple[np.ndarray, np.ndarray]:
-        img = np.empty((nz, nx), np.float32)
-        ill = np.empty((nz, nx), np.float32)
+    def fetch(self, slot: int, nz: int, nx: int, out=None) -> Tuple[np.ndarray, np.ndarray]:
+        """(image, illumination) of a finished migration, into the arrays ``out`` if given."""
+        img, ill = out if out is not None else (np.empty((nz, nx), np.float32),
+                                                np.empty((nz, nx), np.float32))
         _lib.check(self._lib.w2d_batch_fetch(self._h, int(slot), img.ctypes.data, ill.ctypes.data))
         return img, ill
 
@@ -247,11 +248,12 @@ class BatchEngine:
                                                     tr.ctypes.data if tr.size else None))
         return tr
 
-    def collect(self, slot: int, job):
-        """Result of a finished job: (image, illumination) or the modelled gather."""
+    def collect(self, slot: int, job, out=None):
+        """Result of a finished job: (image, illumination), into ``out`` if given, or the
+        modelled gather."""
         if isinstance(job, ModelJob):
             return self.fetch_traces(slot, len(job.wavelet), job.n_receivers)
-        return self.fetch(slot, job.nz, job.nx)
+        return self.fetch(slot, job.nz, job.nx, out)
 
     def run(self, jobs: Sequence) -> Tuple[list, dict]:
         """Run every job (ShotJob or ModelJob, mixed freely; continuous admission);
@@ -259,6 +261,10 @@ class BatchEngine:
         results: List[Optional[Tuple[np.ndarray, np.ndarray]]] = [None] * len(jobs)
         pending = list(range(len(jobs)))
         running: Dict[int, int] = {}
+        # Result arrays of running migrations, made and touched while a replay runs: their
+        # pages are mapped then, not one fault at a time under the copy back, during which
+        # the device has nothing to do (20 gathers: 196 -> 155 ms).
+        ready: Dict[int, Tuple[np.ndarray, np.ndarray]] = {}
         dev_ms = 0.0
         pts = 0.0
         launches = 0
@@ -271,6 +277,18 @@ class BatchEngine:
                     break
                 running[slot] = pending.pop(0)
 
+        def make_ready(limit=1 << 23):
+            for slot, j in running.items():
+                if limit <= 0:
+                    break
+                job = jobs[j]
+                if slot not in ready and isinstance(job, ShotJob):
+                    ready[slot] = (np.empty((job.nz, job.nx), np.float32),
+                                   np.empty((job.nz, job.nx), np.float32))
+                    for a in ready[slot]:
+                        a.fill(0.0)
+                        limit -= a.nbytes
+
         admit()
         flying = False
         while running or pending:
@@ -282,6 +300,7 @@ class BatchEngine:
             if not flying:
                 self.launch()
             admit()  # uploads overlap the replay in flight; these shots join the next one
+            make_ready()
             self.wait()
             dev_ms += self.last_ms
             pts += self.last_points
@@ -293,6 +312,6 @@ class BatchEngine:
                 self.launch()
             for slot in fin:
                 j = running.pop(slot)
-                results[j] = self.collect(slot, jobs[j])
+                results[j] = self.collect(slot, jobs[j], ready.pop(slot, None))
         return results, {"device_ms": dev_ms, "counted_points": pts, "launches": launches,
                          "max_active": max_active}
