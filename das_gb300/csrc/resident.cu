@@ -29,7 +29,9 @@
 //     arithmetic; from the adjacent lanes, by shuffles and selects, they cost ten more
 //     instructions of a hundred.)
 //   * The halo warp collects the neighbours' edges meanwhile into the halo of p_next,
-//     samples the receivers of the last step, and prefetches the next snapshot into L2.
+//     samples the receivers of the last step, stages the next one's injection values from
+//     registers it loaded a step before, and prefetches the next snapshot into L2.  (It runs
+//     a loop of its own: what it keeps from step to step costs the compute warps nothing.)
 // One barrier ends the step.
 //
 // Exchange: 16-byte packets {value, tag, value, tag} in global memory, tag = step
@@ -316,12 +318,24 @@ __device__ __forceinline__ F4 rs_special(const F4& v, int nxt, int row, int c, i
 __device__ __forceinline__ void rs_sample(float* row, int pl, int par)
 {
     const RsTile& t = rs_tile();
-    const int src_x = t.src_row == t.rec_row ? t.src_x : -1;
-    for (int c = threadIdx.x & 31; c < t.pitch; c += 32) {
-        const int r = __float_as_int(rs_smem[t.rk + c]);
-        float v = rs_smem[pl + (t.rec_row + 2) * t.pitch + c];
-        if (c == src_x) v = rs_smem[t.pre + par];  // without the next step's injection
-        if (r >= 0) row[r] = v;
+    const int src_x = t.src_row == t.rec_row ? t.src_x : -1, ncol = t.ncol;
+    const float* at = rs_smem + pl + (t.rec_row + 2) * t.pitch;
+    const float* rk = rs_smem + t.rk;
+    const float before = rs_smem[t.pre + par];  // without the next step's injection
+#pragma unroll 2
+    for (int c = threadIdx.x & 31; c < ncol; c += 32) {  // a unit a lane
+        const int4 r = *reinterpret_cast<const int4*>(rk + 4 * c);
+        float4 v = *reinterpret_cast<const float4*>(at + 4 * c);
+        if (src_x >> 2 == c) {
+            if ((src_x & 3) == 0) v.x = before;
+            if ((src_x & 3) == 1) v.y = before;
+            if ((src_x & 3) == 2) v.z = before;
+            if ((src_x & 3) == 3) v.w = before;
+        }
+        if (r.x >= 0) row[r.x] = v.x;
+        if (r.y >= 0) row[r.y] = v.y;
+        if (r.z >= 0) row[r.z] = v.z;
+        if (r.w >= 0) row[r.w] = v.w;
     }
 }
 
@@ -535,6 +549,20 @@ __device__ __forceinline__ bool rs_collect(const uint4* src, unsigned tag, int n
         }
         if (__any_sync(0xffffffffu, left)) return false;
     }
+}
+
+// The barrier that ends a step, from the compute warps' loop and from the halo warp's; true
+// when a thread of either passes bad.
+__device__ __forceinline__ bool rs_barrier(bool bad, int threads)
+{
+    unsigned r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\t"
+        "barrier.cta.red.or.pred q, 1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(r)
+        : "r"((unsigned)bad), "r"(threads)
+        : "memory");
+    return r != 0;
 }
 
 // many: the launch covers several shots, items[CTA] = {shot, tile}; else the one shot.
@@ -833,14 +861,29 @@ static __global__ void __launch_bounds__(RS_T, 1)
         int ks = (fwd ? ka : 2 * nt - 1 - ka) / s.interval,
             rem = (fwd ? ka : 2 * nt - 1 - ka) - ks * s.interval;
 
+        // one step on: roles, packet tag, this step's place between snapshots
+        auto advance = [&]() {
+            m3 = m3 == 2 ? 0 : m3 + 1;
+            ++tag;
+            par ^= 1;
+            if (fwd) {
+                if (++rem == s.interval) {
+                    rem = 0;
+                    ++ks;
+                }
+            } else if (rem-- == 0) {
+                rem = s.interval - 1;
+                --ks;
+            }
+        };
+        if (!halo) {
 #pragma unroll 1
-        for (int k = ka; k < kb; ++k, par ^= 1) {
-            // nothing derived from the records or from m is kept from step to step: it
-            // would not fit the registers
-            asm volatile("" : "+r"(m.e), "+r"(m.i), "+r"(m.b)::"memory");
-            const int cur = RS_PLANE0 + (par ? dpl : 0), nxt = RS_PLANE0 + (par ? 0 : dpl);
-            const bool on = rem == 0;  // a step with a snapshot
-            if (!halo) {
+            for (int k = ka; k < kb; ++k) {
+                // nothing derived from the records or from m is kept from step to step: it
+                // would not fit the registers
+                asm volatile("" : "+r"(m.e), "+r"(m.i), "+r"(m.b)::"memory");
+                const int cur = RS_PLANE0 + (par ? dpl : 0), nxt = RS_PLANE0 + (par ? 0 : dpl);
+                const bool on = rem == 0;  // a step with a snapshot
                 // ---- phase E
                 if (e_warp) {
                     const int ec = m.ec(), oc = cur + (m.er() + 2) * pitch + 4 * ec;
@@ -881,18 +924,6 @@ static __global__ void __launch_bounds__(RS_T, 1)
                     if (on && fwd && s.lap && m.e_live())
                         rs_snap(s.snaps + (size_t)(ks - s.slot0) * s.plane +
                                     (size_t)(t.z0 + m.er()) * t.ldx + t.x0 + 4 * ec, lap);
-                }
-                // the next step's injection, a column a thread: on its way from here, staged at
-                // the end of the step
-                float nd = -0.0f, nf = 1.0f;
-                const bool stage = !fwd && t.rec_row >= 0 && tid < pitch;
-                if (stage && k + 1 < kb) {
-                    const float* d = data_row(k + 1);
-                    const int r = rec_of(tid);
-                    if (d && r >= 0) {
-                        nd = d[r];
-                        nf = inj_factor(tid);
-                    }
                 }
                 RsFused fu{nullptr, nullptr, false, false, adj_top && m.r0() == 2};
                 if (on) {
@@ -943,25 +974,63 @@ static __global__ void __launch_bounds__(RS_T, 1)
                     }
                     __syncwarp();
                 }
-                if (stage) rs_smem[t.inj + (par ^ 1) * pitch + tid] = fmul(nd, nf);
-                __syncwarp();
-                bad = !rs_collect<2>(s.xbuf + t.in + (tag & 1u) * t.half, tag, nxt, par ^ 1,
+                bad = !rs_collect<RS_FLIGHT_C>(s.xbuf + t.in + (tag & 1u) * t.half, tag, nxt, par ^ 1,
                                      t.next + par, s.err);
-            } else {
-                // ---- halo warp: the last step's samples, the next step's injection, the
-                // next snapshot, the edges
-                if (k > ka && t.rec_row >= 0 && rec_row_out(k - 1))
-                    rs_sample(rec_row_out(k - 1), cur, par ^ 1);
+                advance();
+                if (rs_barrier(bad, RS_T)) {
+                    bad = true;
+                    break;
+                }
+            }
+        } else {
+            // Injection values, a step ahead in registers: what a step adds is loaded during the
+            // step before the last one and staged in the last one (columns lane + 32 j; those
+            // of tiles wider than 256 points past them as they are staged).
+            float nd[8], nf[8], ns = -0.0f;
+            const bool rec = !fwd && t.rec_row >= 0;
+            auto load_injection = [&](int k) {
+                const float* d = k < kb ? data_row(k) : nullptr;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const int c = lane + 32 * j, r = c < pitch ? rec_of(c) : -1;
+                    nd[j] = d && r >= 0 ? d[r] : -0.0f;
+                }
+            };
+            auto load_source = [&](int k) {
+                ns = fwd && t.src_row >= 0 && k < kb && k + 1 < nt ? s.wavelet[k + 1] : -0.0f;
+            };
+            if (rec) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const int c = lane + 32 * j;
+                    nf[j] = c < pitch && rec_of(c) >= 0 ? inj_factor(c) : 1.0f;
+                }
+                load_injection(ka + 1);
+            }
+            load_source(ka + 1);
+#pragma unroll 1
+            for (int k = ka; k < kb; ++k) {
+                const int cur = RS_PLANE0 + (par ? dpl : 0), nxt = RS_PLANE0 + (par ? 0 : dpl);
                 const bool more = k + 1 < kb;
-                if (t.rec_row >= 0)  // columns past the compute threads'
-                    for (int c = RS_CT + lane; c < pitch; c += 32) {
+                if (rec) {
+                    float* inj = rs_smem + t.inj + (par ^ 1) * pitch;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        if (lane + 32 * j < pitch) inj[lane + 32 * j] = fmul(nd[j], nf[j]);
+                    load_injection(k + 2);
+                    for (int c = 256 + lane; c < pitch; c += 32) {
                         const float* d = more ? data_row(k + 1) : nullptr;
                         const int r = rec_of(c);
-                        rs_smem[t.inj + (par ^ 1) * pitch + c] =
-                            d && r >= 0 ? fmul(d[r], inj_factor(c)) : -0.0f;
+                        inj[c] = d && r >= 0 ? fmul(d[r], inj_factor(c)) : -0.0f;
                     }
-                float ns = -0.0f;
-                if (lane == 0 && more) ns = src_value(k + 1);
+                }
+                if (lane == 0) {
+                    rs_smem[t.injs + (par ^ 1)] = fmul(ns, s.dt2_inj);
+                    reinterpret_cast<int*>(rs_smem)[t.next + (par ^ 1)] = 0;
+                }
+                load_source(k + 2);
+                if (k > ka && t.rec_row >= 0 && rec_row_out(k - 1))
+                    rs_sample(rec_row_out(k - 1), cur, par ^ 1);
                 if (!fwd && more && s.image && s.snaps && (rem == 1 || s.interval == 1)) {
                     const int k1 = rem == 0 ? ks - 1 : ks;
                     if (k1 < s.n_snaps)
@@ -970,26 +1039,14 @@ static __global__ void __launch_bounds__(RS_T, 1)
                                                  (size_t)(t.z0 + r) * t.ldx + t.x0,
                                              (uint32_t)t.pitch * 4u);
                 }
-                if (lane == 0) reinterpret_cast<int*>(rs_smem)[t.next + (par ^ 1)] = 0;
                 __syncwarp();
-                bad = !rs_collect<RS_FLIGHT>(s.xbuf + t.in + (tag & 1u) * t.half, tag, nxt,
+                bad = !rs_collect<RS_FLIGHT_H>(s.xbuf + t.in + (tag & 1u) * t.half, tag, nxt,
                                              par ^ 1, t.next + par, s.err);
-                if (lane == 0) rs_smem[t.injs + (par ^ 1)] = ns;
-            }
-            m3 = m3 == 2 ? 0 : m3 + 1;
-            ++tag;
-            if (fwd) {
-                if (++rem == s.interval) {
-                    rem = 0;
-                    ++ks;
+                advance();
+                if (rs_barrier(bad, RS_T)) {
+                    bad = true;
+                    break;
                 }
-            } else if (rem-- == 0) {
-                rem = s.interval - 1;
-                --ks;
-            }
-            if (__syncthreads_or(bad)) {
-                bad = true;
-                break;
             }
         }
 
