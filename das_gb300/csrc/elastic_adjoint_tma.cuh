@@ -4,9 +4,12 @@
 // el_adj_a (K2 + K3 of step n) and el_adj_b (K4 of step n with K1 of step n-1) on
 // 128 x TZ tiles of shot blockIdx.z.  The fields a pass differentiates arrive as
 // 136 x (TZ+4) TMA boxes on one mbarrier (2-row / 4-column halo; outside the grid
-// the boxes read zero, the fields' value outside M): pass A takes the three
-// t = dt C q planes, the forward velocities of u_{n+1} and the forward stresses of
-// u_n (eight boxes); pass B the two r = dt b adj_v planes.  Each lane owns four
+// the boxes read zero, the fields' value outside M): pass A takes the three adjoint
+// stresses q, lambda and mu, the forward velocities of u_{n+1} and the forward stresses
+// of u_n (ten boxes); pass B the two r = dt b adj_v planes.  Pass A forms t = dt C q in
+// its boxes, over the halo too: as planes of their own, written by pass B and read back,
+// t cost six of the 42 planes an adjoint step moved: 1024 x 2048, 500 steps
+// forward and gradient 41.4 -> 39.1 ms.  Each lane owns four
 // consecutive x points (float4), x neighbours come by warp shuffles, z neighbours
 // are read from the box rows; the fields used at one point only (adjoint fields,
 // parameters, gradients) are float4 global accesses.  Arithmetic as the reference
@@ -23,8 +26,8 @@ struct ElAdjTile {
     static constexpr int TZ = WARPS * RPW;
     static constexpr int BOX = (TZ + 4) * EL_SW;
     static constexpr int PT = TZ * EL_TX;              // one staged pointwise field
-    static constexpr int A_FLOATS = 8 * BOX + 12 * PT;  // pass A
-    static constexpr int B_FLOATS = 2 * BOX + 6 * PT;   // pass B
+    static constexpr int A_FLOATS = 10 * BOX + 9 * PT;  // pass A
+    static constexpr int B_FLOATS = 2 * BOX + 4 * PT;   // pass B
 };
 
 // c1*(a[x+1]-a[x]) + c2*(a[x+2]-a[x-1]) of point j from an el_xrow row
@@ -69,7 +72,10 @@ struct ElAdjRecv {
 };
 
 struct ElAdjMaps {
-    CUtensorMap tmp;  // the t / r planes (5 per shot)
+    CUtensorMap tmp;  // the r planes (5 per shot, the velocities' used)
+    CUtensorMap adj;  // the adjoint state (5 per shot)
+    CUtensorMap par;  // the parameters (4 per shot, or 4 in all: par_step planes per shot)
+    int par_step;
     CUtensorMap fwd;  // forward states: u_n's planes from curr0 on, u_{n+1}'s from next0 on
     int next0, curr0;
 };
@@ -83,7 +89,7 @@ __global__ void __launch_bounds__(WARPS * 32)
 {
     using T = ElAdjTile<WARPS, RPW>;
     extern __shared__ __align__(128) float smem[];
-    float* b_txx = smem;
+    float* b_txx = smem;               // q, then t = dt C q, in place
     float* b_txz = smem + T::BOX;
     float* b_tzz = smem + 2 * T::BOX;
     float* b_nvx = smem + 3 * T::BOX;
@@ -91,8 +97,10 @@ __global__ void __launch_bounds__(WARPS * 32)
     float* b_cxx = smem + 5 * T::BOX;
     float* b_cxz = smem + 6 * T::BOX;
     float* b_czz = smem + 7 * T::BOX;
-    // staged: adj vx, vz, sxx, szz, sxz, g_lambda, g_mu, sponge, bx, bz, g_bx, g_bz
-    float* pt = smem + 8 * T::BOX;
+    float* b_lam = smem + 8 * T::BOX;
+    float* b_mu = smem + 9 * T::BOX;
+    // staged: adj vx, vz, g_lambda, g_mu, sponge, bx, bz, g_bx, g_bz
+    float* pt = smem + 10 * T::BOX;
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem + T::A_FLOATS);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int x0 = blockIdx.x * EL_TX, z0 = blockIdx.y * T::TZ, sh = blockIdx.z;
@@ -105,11 +113,13 @@ __global__ void __launch_bounds__(WARPS * 32)
     grid_dep_launch();
     grid_dep_wait();
     if (tid == 0) {
-        mbar_expect_tx(bar, 8u * T::BOX * 4u);
+        mbar_expect_tx(bar, 10u * T::BOX * 4u);
         const int xs = x0 - EL_HX, zs = z0 - 2, pb = 5 * sh;
-        tma_load_3d(b_txx, &maps.tmp, xs, zs, pb + EL_SXX, bar);
-        tma_load_3d(b_txz, &maps.tmp, xs, zs, pb + EL_SXZ, bar);
-        tma_load_3d(b_tzz, &maps.tmp, xs, zs, pb + EL_SZZ, bar);
+        tma_load_3d(b_txx, &maps.adj, xs, zs, pb + EL_SXX, bar);
+        tma_load_3d(b_txz, &maps.adj, xs, zs, pb + EL_SXZ, bar);
+        tma_load_3d(b_tzz, &maps.adj, xs, zs, pb + EL_SZZ, bar);
+        tma_load_3d(b_lam, &maps.par, xs, zs, maps.par_step * sh, bar);
+        tma_load_3d(b_mu, &maps.par, xs, zs, maps.par_step * sh + 1, bar);
         tma_load_3d(b_nvx, &maps.fwd, xs, zs, maps.next0 + pb + EL_VX, bar);
         tma_load_3d(b_nvz, &maps.fwd, xs, zs, maps.next0 + pb + EL_VZ, bar);
         tma_load_3d(b_cxx, &maps.fwd, xs, zs, maps.curr0 + pb + EL_SXX, bar);
@@ -130,9 +140,8 @@ __global__ void __launch_bounds__(WARPS * 32)
     const int zr0 = z0 + warp * RPW;
     const int sr0 = zr0 - (z0 - 2);
     {
-        const float* f[12] = {a.vx, a.vz, a.sxx, a.szz, a.sxz, g_lam, g_mu,
-                              p.sponge, bxp, bzp, g_bx, g_bz};
-        el_stage_pointwise<WARPS, RPW>(pt, f, 12, zr0, ixb, lane, warp, g);
+        const float* f[9] = {a.vx, a.vz, g_lam, g_mu, p.sponge, bxp, bzp, g_bx, g_bz};
+        el_stage_pointwise<WARPS, RPW>(pt, f, 9, zr0, ixb, lane, warp, g);
     }
     __syncthreads();
     if (__syncthreads_or(!mbar_wait_bounded(bar, 0))) {
@@ -142,6 +151,42 @@ __global__ void __launch_bounds__(WARPS * 32)
     }
     cp_async_wait_all();  // this thread's staged fields (read and updated only by it)
     auto staged = [&](int f, int rr) { return el_staged<WARPS, RPW>(pt, f, warp, rr, lane); };
+    // this thread's own q, then t = dt C q over the boxes in place
+    float4 qxx_r[RPW], qzz_r[RPW], qxz_r[RPW];
+#pragma unroll
+    for (int rr = 0; rr < RPW; ++rr) {
+        qxx_r[rr] = el_row4(b_txx, sr0 + rr, lane);
+        qzz_r[rr] = el_row4(b_tzz, sr0 + rr, lane);
+        qxz_r[rr] = el_row4(b_txz, sr0 + rr, lane);
+    }
+    __syncthreads();
+    // t is zero outside M whatever the parameters hold there: only border tiles test it
+    const bool border = x0 - EL_HX < 2 || z0 - 2 < 2 || x0 + EL_TX + EL_HX > g.nx - 2 ||
+                        z0 + T::TZ + 2 > g.nz - 2;
+    for (int i = tid; i < T::BOX / 4; i += WARPS * 32) {
+        float4 *xx = reinterpret_cast<float4*>(b_txx) + i, *zz = reinterpret_cast<float4*>(b_tzz) + i,
+               *xz = reinterpret_cast<float4*>(b_txz) + i;
+        const float4 l4 = reinterpret_cast<const float4*>(b_lam)[i],
+                     m4 = reinterpret_cast<const float4*>(b_mu)[i], qx = *xx, qz = *zz, qs = *xz;
+        float ox[4], oz[4], os[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            float l = el_c(l4, j), m = el_c(m4, j);
+            const float x = el_c(qx, j), zv = el_c(qz, j);
+            if (border) {
+                const int row = i / (EL_SW / 4), col = 4 * (i - row * (EL_SW / 4)) + j;
+                if (!el_in_m(x0 - EL_HX + col, z0 - 2 + row, g.nx, g.nz, g.free_surface))
+                    l = m = 0.0f;
+            }
+            ox[j] = g.dt * ((l + 2.0f * m) * x + l * zv);
+            oz[j] = g.dt * (l * x + (l + 2.0f * m) * zv);
+            os[j] = g.dt * m * el_c(qs, j);
+        }
+        *xx = make_float4(ox[0], ox[1], ox[2], ox[3]);
+        *zz = make_float4(oz[0], oz[1], oz[2], oz[3]);
+        *xz = make_float4(os[0], os[1], os[2], os[3]);
+    }
+    __syncthreads();
     if (rv.resid && col_ok && zr0 + RPW > rv.rec_iz - 2 && zr0 <= rv.rec_iz + 1) {
         // the receivers' residuals on the four rows of their strain stencil (each cell's
         // contributions in receiver order), added to this thread's staged adjoint vz
@@ -166,7 +211,7 @@ __global__ void __launch_bounds__(WARPS * 32)
         }
     }
     // Two phases per row (K2, then K3) so that only one phase's operands are live.
-#pragma unroll 1
+#pragma unroll
     for (int rr = 0; rr < RPW; ++rr) {
         const int iz = zr0 + rr, sr = sr0 + rr;
         const bool live = iz < g.nz && col_ok;
@@ -199,8 +244,8 @@ __global__ void __launch_bounds__(WARPS * 32)
                              nvz_m1 = el_row4(b_nvz, sr - 1, lane),
                              nvz_p1 = el_row4(b_nvz, sr + 1, lane);
                 const float4 avx4 = staged(0, rr), avz4 = staged(1, rr);
-                const float4 qxx4 = staged(2, rr), qzz4 = staged(3, rr), qxz4 = staged(4, rr);
-                const float4 gl4 = staged(5, rr), gm4 = staged(6, rr);
+                const float4 qxx4 = qxx_r[rr], qzz4 = qzz_r[rr], qxz4 = qxz_r[rr];
+                const float4 gl4 = staged(2, rr), gm4 = staged(3, rr);
                 float o_gl[4], o_gm[4];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
@@ -249,9 +294,9 @@ __global__ void __launch_bounds__(WARPS * 32)
                 const float4 czz_m1 = el_row4(b_czz, sr - 1, lane), czz_c = el_row4(b_czz, sr, lane),
                              czz_p1 = el_row4(b_czz, sr + 1, lane),
                              czz_p2 = el_row4(b_czz, sr + 2, lane);
-                const float4 sp4 = p.sponge ? staged(7, rr) : make_float4(1.f, 1.f, 1.f, 1.f);
-                const float4 bx4 = staged(8, rr), bz4 = staged(9, rr);
-                const float4 gbx4 = staged(10, rr), gbz4 = staged(11, rr);
+                const float4 sp4 = p.sponge ? staged(4, rr) : make_float4(1.f, 1.f, 1.f, 1.f);
+                const float4 bx4 = staged(5, rr), bz4 = staged(6, rr);
+                const float4 gbx4 = staged(7, rr), gbz4 = staged(8, rr);
                 float o_gbx[4], o_gbz[4], o_rx[4], o_rz[4];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
@@ -294,17 +339,17 @@ __global__ void __launch_bounds__(WARPS * 32)
     }
 }
 
-// K4 of step n, then (then_k1) K1 of step n-1
+// K4 of step n, then (then_k1) the sponge of step n-1 (K1's q; pass A forms its t)
 template <int WARPS, int RPW>
 __global__ void __launch_bounds__(WARPS * 32)
     el_adj_b(const __grid_constant__ ElAdjMaps maps, const ElGeom g, const ElParams p,
-             const ElStrides sd, ElState a, ElState t, int then_k1, unsigned* err)
+             const ElStrides sd, ElState a, int then_k1, unsigned* err)
 {
     using T = ElAdjTile<WARPS, RPW>;
     extern __shared__ __align__(128) float smem[];
     float* b_rx = smem;
     float* b_rz = smem + T::BOX;
-    float* pt = smem + 2 * T::BOX;  // staged adj sxx, szz, sxz, sponge, lambda, mu
+    float* pt = smem + 2 * T::BOX;  // staged adj sxx, szz, sxz, sponge
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem + T::B_FLOATS);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int x0 = blockIdx.x * EL_TX, z0 = blockIdx.y * T::TZ, sh = blockIdx.z;
@@ -321,17 +366,12 @@ __global__ void __launch_bounds__(WARPS * 32)
     }
     const int ixb = x0 + 4 * lane;
     const bool col_ok = ixb < g.ldx;
-    const size_t so = (size_t)sh * sd.state, po = (size_t)sh * sd.param;
-    a = el_shift(a, so);
-    t = el_shift(t, so);
-    const float* lamp = p.lam + po;
-    const float* mup = p.mu + po;
+    a = el_shift(a, (size_t)sh * sd.state);
     const int zr0 = z0 + warp * RPW;
     const int sr0 = zr0 - (z0 - 2);
     {
-        const float* f[6] = {a.sxx, a.szz, a.sxz, then_k1 ? p.sponge : nullptr,
-                             then_k1 ? lamp : nullptr, then_k1 ? mup : nullptr};
-        el_stage_pointwise<WARPS, RPW>(pt, f, 6, zr0, ixb, lane, warp, g);
+        const float* f[4] = {a.sxx, a.szz, a.sxz, then_k1 ? p.sponge : nullptr};
+        el_stage_pointwise<WARPS, RPW>(pt, f, 4, zr0, ixb, lane, warp, g);
     }
     __syncthreads();
     if (__syncthreads_or(!mbar_wait_bounded(bar, 0))) {
@@ -355,13 +395,9 @@ __global__ void __launch_bounds__(WARPS * 32)
         const float4 sxx4 = el_staged<WARPS, RPW>(pt, 0, warp, rr, lane),
                      szz4 = el_staged<WARPS, RPW>(pt, 1, warp, rr, lane),
                      sxz4 = el_staged<WARPS, RPW>(pt, 2, warp, rr, lane);
-        float4 sp4 = make_float4(1.f, 1.f, 1.f, 1.f), l4 = sp4, m4 = sp4;
-        if (then_k1) {
-            if (p.sponge) sp4 = el_staged<WARPS, RPW>(pt, 3, warp, rr, lane);
-            l4 = el_staged<WARPS, RPW>(pt, 4, warp, rr, lane);
-            m4 = el_staged<WARPS, RPW>(pt, 5, warp, rr, lane);
-        }
-        float oxx[4], ozz[4], oxz[4], txx[4], tzz[4], txz[4];
+        float4 sp4 = make_float4(1.f, 1.f, 1.f, 1.f);
+        if (then_k1 && p.sponge) sp4 = el_staged<WARPS, RPW>(pt, 3, warp, rr, lane);
+        float oxx[4], ozz[4], oxz[4];
         bool all = true;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -371,30 +407,15 @@ __global__ void __launch_bounds__(WARPS * 32)
             szz -= adj_dzm(el_c(rz_m2, j), el_c(rz_m1, j), erz[j + 2], el_c(rz_p1, j)) * g.rdz;
             sxz -= adj_dzp(el_c(rx_m1, j), erx[j + 2], el_c(rx_p1, j), el_c(rx_p2, j)) * g.rdz +
                    adj_dxp(erz, j) * g.rdx;
-            txx[j] = tzz[j] = txz[j] = 0.0f;
-            if (then_k1) {
-                const float sp = el_c(sp4, j);
-                sxx = sp * sxx;
-                szz = sp * szz;
-                sxz = sp * sxz;
-                const float l = el_c(l4, j), m = el_c(m4, j);
-                txx[j] = g.dt * ((l + 2.0f * m) * sxx + l * szz);
-                tzz[j] = g.dt * (l * sxx + (l + 2.0f * m) * szz);
-                txz[j] = g.dt * m * sxz;
-            }
-            oxx[j] = sxx;
-            ozz[j] = szz;
-            oxz[j] = sxz;
+            const float sp = el_c(sp4, j);
+            oxx[j] = sp * sxx;
+            ozz[j] = sp * szz;
+            oxz[j] = sp * sxz;
         }
         if (all) {
             st4(a.sxx + off, oxx);
             st4(a.szz + off, ozz);
             st4(a.sxz + off, oxz);
-            if (then_k1) {
-                st4(t.sxx + off, txx);
-                st4(t.szz + off, tzz);
-                st4(t.sxz + off, txz);
-            }
         } else {
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
@@ -403,11 +424,6 @@ __global__ void __launch_bounds__(WARPS * 32)
                 a.sxx[c] = oxx[j];
                 a.szz[c] = ozz[j];
                 a.sxz[c] = oxz[j];
-                if (then_k1) {
-                    t.sxx[c] = txx[j];
-                    t.szz[c] = tzz[j];
-                    t.sxz[c] = txz[j];
-                }
             }
         }
     }
@@ -437,8 +453,8 @@ cudaError_t launch_el_adj_a_t(const ElAdjMaps& m, const ElGeom& g, const ElParam
 
 template <int WARPS, int RPW>
 cudaError_t launch_el_adj_b_t(const ElAdjMaps& m, const ElGeom& g, const ElParams& p,
-                              const ElStrides& sd, const ElState& a, const ElState& t,
-                              int then_k1, unsigned* err, int n_shots, cudaStream_t st, int pdl)
+                              const ElStrides& sd, const ElState& a, int then_k1, unsigned* err,
+                              int n_shots, cudaStream_t st, int pdl)
 {
     using T = ElAdjTile<WARPS, RPW>;
     const int bytes = T::B_FLOATS * 4 + 128;
@@ -446,7 +462,7 @@ cudaError_t launch_el_adj_b_t(const ElAdjMaps& m, const ElGeom& g, const ElParam
     if (e != cudaSuccess) return e;
     dim3 grid((g.nx + EL_TX - 1) / EL_TX, (g.nz + T::TZ - 1) / T::TZ, n_shots);
     return el_launch(el_adj_b<WARPS, RPW>, grid, dim3(WARPS * 32), bytes, st, pdl, m, g, p, sd, a,
-                     t, then_k1, err);
+                     then_k1, err);
 }
 
 // Pass A / pass B on tiles of `warps` x `rpw` rows (maps with box height warps*rpw + 4).
@@ -470,16 +486,16 @@ inline cudaError_t launch_el_adj_a(const ElAdjMaps& m, const ElGeom& g, const El
 }
 
 inline cudaError_t launch_el_adj_b(const ElAdjMaps& m, const ElGeom& g, const ElParams& p,
-                                   const ElStrides& sd, const ElState& a, const ElState& t,
-                                   int then_k1, unsigned* err, int n_shots, cudaStream_t st,
+                                   const ElStrides& sd, const ElState& a, int then_k1,
+                                   unsigned* err, int n_shots, cudaStream_t st,
                                    int warps = EL_ADJ_WARPS, int rpw = EL_ADJ_RPW, int pdl = 0)
 {
     if (warps == 4 && rpw == 2)
-        return launch_el_adj_b_t<4, 2>(m, g, p, sd, a, t, then_k1, err, n_shots, st, pdl);
+        return launch_el_adj_b_t<4, 2>(m, g, p, sd, a, then_k1, err, n_shots, st, pdl);
     if (warps == 4 && rpw == 1)
-        return launch_el_adj_b_t<4, 1>(m, g, p, sd, a, t, then_k1, err, n_shots, st, pdl);
+        return launch_el_adj_b_t<4, 1>(m, g, p, sd, a, then_k1, err, n_shots, st, pdl);
     if (warps == 8 && rpw == 1)
-        return launch_el_adj_b_t<8, 1>(m, g, p, sd, a, t, then_k1, err, n_shots, st, pdl);
+        return launch_el_adj_b_t<8, 1>(m, g, p, sd, a, then_k1, err, n_shots, st, pdl);
     return cudaErrorInvalidValue;
 }
 

@@ -77,6 +77,7 @@ struct w2d_elastic {
     int pdl = 1;
     bool chain = false;
     bool last_stress = false;  // ... and that kernel was a stress phase
+    CUtensorMap adj_map_adj, adj_map_par;
     CUtensorMap adj_map_tmp;                // the adjoint passes' maps (their own box height)
     CUtensorMap adj_map_seg;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -341,7 +342,10 @@ int w2d_elastic_forward_batch(w2d_elastic* e, int n_shots, const float* lam, con
     const int n_states = S * (e->seg_len + 1);
     if ((rc = make_el_state_map(&e->map_seg, e->seg, e->nx, e->nz, e->ldx, P, n_states, ftz)) ||
         (rc = make_el_adj_map(&e->adj_map_seg, e->seg, e->nx, e->nz, e->ldx, P, n_states, atz)) ||
-        (rc = make_el_adj_map(&e->adj_map_tmp, e->tmp, e->nx, e->nz, e->ldx, P, S, atz)))
+        (rc = make_el_adj_map(&e->adj_map_tmp, e->tmp, e->nx, e->nz, e->ldx, P, S, atz)) ||
+        (rc = make_el_adj_map(&e->adj_map_adj, e->adj, e->nx, e->nz, e->ldx, P, S, atz)) ||
+        (rc = make_tensor_map_3d(&e->adj_map_par, e->params, e->nx, e->nz, 4 * S, e->ldx, P, EL_SW,
+                                 atz + 4)))
         return rc;
     const size_t hp = (size_t)e->nx * 4, dp = (size_t)e->ldx * 4, np = (size_t)e->nx * e->nz;
     const float* src[4] = {lam, mu, bx, bz};
@@ -462,6 +466,9 @@ int w2d_elastic_gradient_batch(w2d_elastic* e, const float* resid_dev, float* g_
             if (e->adj_form == 1) {
                 ElAdjMaps m;
                 m.tmp = e->adj_map_tmp;
+                m.adj = e->adj_map_adj;
+                m.par = e->adj_map_par;
+                m.par_step = e->pstride ? 4 : 0;
                 m.fwd = e->adj_map_seg;
                 m.next0 = 5 * S * (n + 1 - a0);
                 m.curr0 = 5 * S * (n - a0);
@@ -470,7 +477,7 @@ int w2d_elastic_gradient_batch(w2d_elastic* e, const float* resid_dev, float* g_
                 W2D_CUDA_TRY(launch_el_adj_a(m, g, prm, sd, a, r, glam, gmu, gbx, gbz, rv, e->err,
                                              S, e->st, e->map_adj_warps, e->map_adj_rpw,
                                              e->pdl && e->chain));
-                W2D_CUDA_TRY(launch_el_adj_b(m, g, prm, sd, a, t, n >= 1 ? 1 : 0, e->err, S,
+                W2D_CUDA_TRY(launch_el_adj_b(m, g, prm, sd, a, n >= 1 ? 1 : 0, e->err, S,
                                              e->st, e->map_adj_warps, e->map_adj_rpw, e->pdl));
                 e->chain = true;
                 e->last_stress = false;
