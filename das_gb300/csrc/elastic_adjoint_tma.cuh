@@ -26,7 +26,7 @@ struct ElAdjTile {
     static constexpr int TZ = WARPS * RPW;
     static constexpr int BOX = (TZ + 4) * EL_SW;
     static constexpr int PT = TZ * EL_TX;              // one staged pointwise field
-    static constexpr int A_FLOATS = 10 * BOX + 9 * PT;  // pass A
+    static constexpr int A_FLOATS = 10 * BOX + 5 * PT;  // pass A
     static constexpr int B_FLOATS = 2 * BOX + 4 * PT;   // pass B
 };
 
@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(WARPS * 32)
     float* b_czz = smem + 7 * T::BOX;
     float* b_lam = smem + 8 * T::BOX;
     float* b_mu = smem + 9 * T::BOX;
-    // staged: adj vx, vz, g_lambda, g_mu, sponge, bx, bz, g_bx, g_bz
+    // staged: adj vx, vz, sponge, bx, bz
     float* pt = smem + 10 * T::BOX;
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem + T::A_FLOATS);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -140,8 +140,20 @@ __global__ void __launch_bounds__(WARPS * 32)
     const int zr0 = z0 + warp * RPW;
     const int sr0 = zr0 - (z0 - 2);
     {
-        const float* f[9] = {a.vx, a.vz, g_lam, g_mu, p.sponge, bxp, bzp, g_bx, g_bz};
-        el_stage_pointwise<WARPS, RPW>(pt, f, 9, zr0, ixb, lane, warp, g);
+        const float* f[5] = {a.vx, a.vz, p.sponge, bxp, bzp};
+        el_stage_pointwise<WARPS, RPW>(pt, f, 5, zr0, ixb, lane, warp, g);
+    }
+    // The gradients so far wait in registers, which this kernel has to spare: with the
+    // other four fields staged too a CTA took 62 KB and three fitted an SM, not four.
+    float4 gr[RPW][4];
+#pragma unroll
+    for (int rr = 0; rr < RPW; ++rr) {
+        const bool live = zr0 + rr < g.nz && col_ok;
+        const size_t off = (size_t)(zr0 + rr) * g.ldx + ixb;
+        const float* gp[4] = {g_lam, g_mu, g_bx, g_bz};
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            gr[rr][k] = live ? ld4(gp[k] + off) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     __syncthreads();
     if (__syncthreads_or(!mbar_wait_bounded(bar, 0))) {
@@ -245,7 +257,7 @@ __global__ void __launch_bounds__(WARPS * 32)
                              nvz_p1 = el_row4(b_nvz, sr + 1, lane);
                 const float4 avx4 = staged(0, rr), avz4 = staged(1, rr);
                 const float4 qxx4 = qxx_r[rr], qzz4 = qzz_r[rr], qxz4 = qxz_r[rr];
-                const float4 gl4 = staged(2, rr), gm4 = staged(3, rr);
+                const float4 gl4 = gr[rr][0], gm4 = gr[rr][1];
                 float o_gl[4], o_gm[4];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
@@ -294,9 +306,9 @@ __global__ void __launch_bounds__(WARPS * 32)
                 const float4 czz_m1 = el_row4(b_czz, sr - 1, lane), czz_c = el_row4(b_czz, sr, lane),
                              czz_p1 = el_row4(b_czz, sr + 1, lane),
                              czz_p2 = el_row4(b_czz, sr + 2, lane);
-                const float4 sp4 = p.sponge ? staged(4, rr) : make_float4(1.f, 1.f, 1.f, 1.f);
-                const float4 bx4 = staged(5, rr), bz4 = staged(6, rr);
-                const float4 gbx4 = staged(7, rr), gbz4 = staged(8, rr);
+                const float4 sp4 = p.sponge ? staged(2, rr) : make_float4(1.f, 1.f, 1.f, 1.f);
+                const float4 bx4 = staged(3, rr), bz4 = staged(4, rr);
+                const float4 gbx4 = gr[rr][2], gbz4 = gr[rr][3];
                 float o_gbx[4], o_gbz[4], o_rx[4], o_rz[4];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
