@@ -29,7 +29,8 @@
 // .f32x2 pairs of neighbouring lags, half the issue slots for the same pipe time.
 // Measured, one window of 3000 samples, 16 sources, 95 receivers, 351 lags, four windows
 // from creation to read-back: 2.85 ms with scalar operations, 2.44 paired; one source alone
-// 0.69 and 0.49 (whole gather, with one allocation in place of eight).
+// 0.69 and 0.49 (whole gather, with one allocation in place of eight; 0.30 with the block of
+// a handle before it, and 0.14 in place of 0.33 for the correlation of 500 samples).
 #include <math.h>
 #include <string.h>
 
@@ -131,9 +132,10 @@ __global__ void __launch_bounds__(XC_RX * XC_TP)
 {
     __shared__ float4 s_src[XC_CHUNK];  // {s, s, -s, -s}
     __shared__ float s_part[XC_TP][2][XC_LG][XC_RX];  // the parts' (hi, lo) sums
-    const int r = blockIdx.x * XC_RX + threadIdx.x;
+    const int n_rx = (n_rec + XC_RX - 1) / XC_RX;  // blockIdx.x: receivers fastest, then lags
+    const int r = (int)(blockIdx.x % n_rx) * XC_RX + threadIdx.x;
     const int part = threadIdx.y;
-    const int row0 = blockIdx.y * XC_LG;
+    const int row0 = (int)(blockIdx.x / n_rx) * XC_LG;
     const int s = blockIdx.z;
     const float* Ss = S + (size_t)s * nt;
     const int rr = min(r, n_rec - 1);  // lanes past the last receiver compute a copy
@@ -388,6 +390,85 @@ int scratch_stream()
 
 }  // namespace
 
+namespace {
+
+// Blocks of destroyed handles, for the next ones: mapping and unmapping a block's memory
+// takes longer than a short gather's correlation.  A handle gives its block back after its
+// streams have finished, and a new one clears what it does not write, so blocks pass between
+// streams and threads.  Bounded: at most XC_KEPT blocks a device, of at most XC_KEPT_BYTES
+// each, and none is kept when an allocation fails.
+constexpr int XC_KEPT = 2;
+constexpr size_t XC_KEPT_BYTES = (size_t)16 << 20;
+
+struct XcBlocks {
+    struct Block {
+        int device;
+        char* p;
+        size_t size;
+    };
+    std::mutex m;
+    std::vector<Block> kept;
+
+    // a block of the current device `device`, of at least `need` bytes; null without memory
+    char* take(int device, size_t need, size_t* size)
+    {
+        std::lock_guard<std::mutex> lock(m);
+        for (size_t i = 0; i < kept.size(); ++i)
+            if (kept[i].device == device && kept[i].size >= need) {
+                const Block b = kept[i];
+                kept.erase(kept.begin() + i);
+                *size = b.size;
+                return b.p;
+            }
+        char* p = nullptr;
+        if (cudaMalloc(&p, need) != cudaSuccess) {
+            cudaGetLastError();
+            p = nullptr;
+            for (size_t i = 0; i < kept.size();)
+                if (kept[i].device == device) {
+                    cudaFree(kept[i].p);
+                    kept.erase(kept.begin() + i);
+                } else {
+                    ++i;
+                }
+            if (cudaMalloc(&p, need) != cudaSuccess) {
+                cudaGetLastError();
+                return nullptr;
+            }
+        }
+        *size = need;
+        return p;
+    }
+
+    // of several small blocks the larger ones stay
+    void give(int device, char* p, size_t size)
+    {
+        std::lock_guard<std::mutex> lock(m);
+        if (size <= XC_KEPT_BYTES) {
+            kept.push_back(Block{device, p, size});
+            int n = 0;
+            size_t least = kept.size();
+            for (size_t i = 0; i < kept.size(); ++i)
+                if (kept[i].device == device) {
+                    ++n;
+                    if (least == kept.size() || kept[i].size < kept[least].size) least = i;
+                }
+            if (n <= XC_KEPT) return;
+            p = kept[least].p;
+            kept.erase(kept.begin() + least);
+        }
+        cudaFree(p);
+    }
+};
+
+XcBlocks& xc_blocks()
+{
+    static XcBlocks* b = new XcBlocks;  // outlives every handle, also at exit
+    return *b;
+}
+
+}  // namespace
+
 struct w2d_xcorr {
     int device = 0;  // CUDA device current at creation: every call on the handle runs there
     int nt = 0, n_ch = 0, n_src = 0, n_rec = 0, lag0 = 0, n_rows = 0, pad = 0, n_added = 0;
@@ -404,6 +485,7 @@ struct w2d_xcorr {
     float* d_stack = nullptr; // (n_src, n_rows, n_rec)
     float* d_out = nullptr;   // read-back staging
     char* block = nullptr;    // the one allocation that holds all of them
+    size_t block_size = 0;
     cudaStream_t st = nullptr;
 };
 
@@ -462,8 +544,7 @@ int w2d_xcorr_create(w2d_xcorr** out, int nt, int n_ch, const int* src_ch, int n
         set_error("stream/event creation failed");
         return fail(W2D_ECUDA);
     }
-    // one allocation for all buffers (eight of them took longer than a short window's
-    // correlation)
+    // one block for all buffers
     const size_t n_out = (size_t)n_src * std::max(1, x->n_rows) * n_rec;
     size_t total = 0;
     auto place = [&](size_t elements) {
@@ -474,8 +555,7 @@ int w2d_xcorr_create(w2d_xcorr** out, int nt, int n_ch, const int* src_ch, int n
     const size_t o_src = place(n_src), o_rec = place(n_rec), o_d0 = place((size_t)nt * n_ch),
                  o_d1 = place((size_t)nt * n_ch), o_s = place((size_t)n_src * nt),
                  o_r = place((size_t)r_rows * n_rec), o_stack = place(n_out), o_out = place(n_out);
-    if (cudaMalloc(&x->block, total) != cudaSuccess) {
-        cudaGetLastError();
+    if (!(x->block = xc_blocks().take(x->device, total, &x->block_size))) {
         set_error("device allocation failed");
         return fail(W2D_ENOMEM);
     }
@@ -506,9 +586,13 @@ void w2d_xcorr_destroy(w2d_xcorr* x)
 {
     W2D_ON_DEVICE_OF(x);
     if (!x) return;
-    if (x->st) cudaStreamSynchronize(x->st);
-    if (x->st_copy) cudaStreamSynchronize(x->st_copy);
-    if (x->block) cudaFree(x->block);
+    bool done = true;
+    if (x->st) done &= cudaStreamSynchronize(x->st) == cudaSuccess;
+    if (x->st_copy) done &= cudaStreamSynchronize(x->st_copy) == cudaSuccess;
+    if (x->block && done)
+        xc_blocks().give(x->device, x->block, x->block_size);
+    else if (x->block)
+        cudaFree(x->block);
     for (cudaEvent_t ev : x->gathered)
         if (ev) cudaEventDestroy(ev);
     if (x->st_copy) cudaStreamDestroy(x->st_copy);
@@ -535,7 +619,9 @@ int w2d_xcorr_add_device(w2d_xcorr* x, const float* data_dev, int nt)
     // the reference's stack (ndarray +=) needs every window's correlation rows to agree
     W2D_CHECK_ARG(lag0 == x->lag0 && n_rows == x->n_rows,
                   "this window's correlation rows differ from the stack's");
-    W2D_CHECK_ARG((x->n_rows + XC_LG - 1) / XC_LG <= 65535 && x->n_src <= 65535,
+    const long long n_rx = (x->n_rec + XC_RX - 1) / XC_RX,
+                    n_lg = (x->n_rows + XC_LG - 1) / XC_LG;
+    W2D_CHECK_ARG(n_rx * n_lg <= 0x7fffffff && n_lg <= 2 * 65535 && x->n_src <= 65535,
                   "too many lags or sources for one launch");
     if (x->n_rows > 0) {
         if (x->last_nt > nt)  // rows of a longer previous window must read as zero again
@@ -544,7 +630,7 @@ int w2d_xcorr_add_device(w2d_xcorr* x, const float* data_dev, int nt)
         xc_gather_kernel<<<grid_1d((size_t)nt * (x->n_rec + x->n_src)), 256, 0, x->st>>>(
             data_dev, nt, x->n_ch, x->d_src, x->n_src, x->d_rec, x->n_rec, x->pad, x->d_s,
             x->d_r);
-        dim3 grid((x->n_rec + XC_RX - 1) / XC_RX, (x->n_rows + XC_LG - 1) / XC_LG, x->n_src);
+        dim3 grid((unsigned)(n_rx * n_lg), 1, x->n_src);
         xc_kernel<<<grid, dim3(XC_RX, XC_TP), 0, x->st>>>(x->d_s, x->d_r, nt, x->n_rec, x->pad,
                                                           x->lag0, x->n_rows, x->d_stack,
                                                           x->n_added == 0 ? 1 : 0, -0.0f);
