@@ -870,9 +870,12 @@ int w2d_engine_create(w2d_engine** out, int nx, int nz, float dx, float dz, doub
     if ((rc = ensure_tensor_maps(e))) return fail(rc);
     if (!e->use_arr && (!e->use_lut || lut_ok)) {
         e->rs = rs_plans(nx, nz, rs_capacity()).back();
-        if (e->rs.ok() && ((rc = e->rs_x.ensure(e->rs.xbuf_bytes() / sizeof(uint4))) ||
-                           cudaMemset(e->rs_x.p, 0, e->rs.xbuf_bytes()) != cudaSuccess))
-            return fail(rc ? rc : W2D_ECUDA);
+        // without memory for the packets (a few MB) the step kernels run
+        if (e->rs.ok() && (e->rs_x.ensure(e->rs.xbuf_bytes() / sizeof(uint4)) ||
+                           cudaMemset(e->rs_x.p, 0, e->rs.xbuf_bytes()) != cudaSuccess)) {
+            cudaGetLastError();
+            e->rs = RsPlan{};
+        }
     }
     if (cudaDeviceSynchronize() != cudaSuccess) {
         set_error("engine set-up failed");
