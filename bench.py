@@ -15,9 +15,9 @@ per shot (forward + backward; recomputation not counted).
   in page-locked memory; the host->device copies of the gather, wavelet and both
   velocity models and the device->host copies of image and illumination are
   inside the timed region.
-* ``roofline``: the fused step kernel, algorithmic bytes of all step launches in
-  the timed region over the device time of the region, against the measured HBM
-  copy bandwidth.
+* ``roofline``: the algorithmic bytes of all time steps in the timed region over the
+  device time of the region, against the measured HBM copy bandwidth; per launch where
+  each step is one, per step where one launch runs a whole pass on chip.
 * ``cpu_baseline``: the reference's CPU path (wave2d.c + its Python time loops,
   restated in oracle/) timed on this host's cores over a bounded sample.
 * ``--impl reference``: that CPU implementation alone, each step a bounded sample
@@ -119,11 +119,11 @@ def measured_peaks():
     return 6800.0, "fallback"
 
 
-def committed_traffic(key="traffic_bytes_per_launch"):
+def committed_traffic(key="traffic_bytes_per_launch", profile="acoustic_step_large_plain.md"):
     """Per-launch DRAM bytes of the step kernel from the committed ncu summary, or None:
     `traffic_bytes_per_launch` in the live (warm-cache) regime, `cold_traffic_bytes_per_launch`
     with the caches flushed before each launch."""
-    p = os.path.join(REPO, "profiles", "acoustic_step_large_plain.md")
+    p = os.path.join(REPO, "profiles", profile)
     if not os.path.exists(p):
         return None
     with open(p) as f:
@@ -407,13 +407,15 @@ def run_ours(args, dist):
     pts = sv.counted_points_per_shot()
     value = pts * K * dist.world / dev_s / 1e9
 
-    # roofline of the fused step kernel over the timed region
+    # roofline of the time steps over the timed region
     peak, peak_kind = measured_peaks()
     step_launches_per_shot = 2 * sv.nt + recompute // max(K, 1)
+    on_chip = launches < 2 * sv.nt  # one launch advanced many steps
     algo_bytes = bytes_per_shot(sv, interval) * K + recompute * sv.nz * sv.nx * 16
     achieved = algo_bytes / (ms.value / 1e3) / 1e9
     per_launch = algo_bytes / (step_launches_per_shot * K)
-    traffic = committed_traffic()
+    traffic = (committed_traffic("traffic_bytes_per_step", "resident_loop_large.md") if on_chip
+               else committed_traffic())
 
     # end-to-end through the public drop-in call, inputs in page-locked host memory
     ke = max(1, min(K, args.e2e_steps))
@@ -471,16 +473,25 @@ def run_ours(args, dist):
                "device_memory_in_use_gb": (total_b - free_b) / 1e9,
                "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                             "frac": achieved / peak, "traffic": traffic,
-                            "traffic_cold": committed_traffic("cold_traffic_bytes_per_launch"),
-                            "limiter": "latency: the three wave planes and the model (64 MB) "
+                            "traffic_cold": (None if on_chip else
+                                             committed_traffic("cold_traffic_bytes_per_launch")),
+                            "limiter": "issue slots: the wavefields and the model stay in "
+                                       "shared and tensor memory for a whole pass, so DRAM "
+                                       "carries the snapshots alone (traffic: per step); frac is "
+                                       "the bytes a launch per step would move over the HBM "
+                                       "copy rate" if on_chip else
+                                       "latency: the three wave planes and the model (64 MB) "
                                        "stay in L2 from step to step, so DRAM carries the "
                                        "snapshot stream and write-backs (traffic: warm-cache "
                                        "ncu, per launch) and each CTA waits on its own TMA "
                                        "round trip; frac is algorithmic bytes over the HBM "
                                        "copy rate",
                             "peak_source": f"{peak_kind} hbm_gbs",
-                            "kernel": "acoustic_step_kernel (fused forward / backward+imaging)",
-                            "algorithmic_bytes_per_launch": per_launch},
+                            "kernel": ("acoustic_resident_kernel (a whole pass per launch)" if on_chip else
+                                       "acoustic_step_kernel (fused forward / backward+imaging)"),
+                            "algorithmic_bytes_per_launch": (
+                                algo_bytes / max(launches, 1) if on_chip else per_launch),
+                            "algorithmic_bytes_per_step": per_launch},
                "e2e": {"value": e2e, "unit": UNIT, "h2d_bytes_per_step": int(h2d),
                        "d2h_bytes_per_step": int(d2h), "steps": ke,
                        "per_call_ms": [round(c, 2) for c, _ in calls],
@@ -715,9 +726,9 @@ def run_elastic(args, dist):
     # roofline of the gradient phase (the device time of J.backward): per time step and
     # grid point the recomputation moves 56 B (the forward step: five fields read and
     # written, lambda, mu and the two buoyancies read) + 20 B (the five fields stored
-    # into the segment), and the two tiled adjoint passes 28 + 14 planes = 168 B
+    # into the segment), and the two tiled adjoint passes 27 + 9 planes = 144 B
     peak, peak_kind = measured_peaks()
-    grad_bytes = nz * nx * nt * (56 + 20 + 168)
+    grad_bytes = nz * nx * nt * (56 + 20 + 144)
     achieved = grad_bytes / (statistics.mean(grad_ms) / 1e3) / 1e9
     fwd_achieved = nz * nx * nt * 56 / (statistics.mean(fwd_ms) / 1e3) / 1e9
     out = {"metric": "elastic RTM gradient Gpts/s", "value": pts * K / sum(times) / 1e9,
@@ -736,7 +747,7 @@ def run_elastic(args, dist):
                         "peak_source": f"{peak_kind} hbm_gbs",
                         "kernel": "gradient phase: el_adj_a + el_adj_b (tiled adjoint passes) "
                                   "and the segment recomputation's step kernels",
-                        "algorithmic_bytes_per_step_point": 56 + 20 + 168,
+                        "algorithmic_bytes_per_step_point": 56 + 20 + 144,
                         "forward_phase_achieved_gbs": fwd_achieved,
                         "forward_phase_frac": fwd_achieved / peak}}
     _emit(out)

@@ -11,10 +11,10 @@
 // Why: one launch per step reloads every operand (16 bytes a point) from L2 or HBM and
 // pays the fixed chain of a launch, about 6 us, each step.  Here a step costs its
 // arithmetic, and the exchange of a tile's edge hides behind the tile's interior.
-// Measured on GB300, us per step, one launch per step -> here: 150 x 400 5.6 -> 1.9
-// forward, 6.2 -> 2.2 in a migration; 301 x 1203 5.8 -> 2.3, 6.5 -> 2.8; 600 x 2000 6.9 ->
-// 3.3, 7.6 -> 5.2; 1000 x 4000 11.2 -> 5.5, 13.4 -> 7.9 (506 Gpts/s).  Small grids are
-// bound by the chain edge -> packet -> neighbour's halo (about 1.8 us), large ones by
+// Measured on GB300, us per step, one launch per step -> here: 150 x 400 5.6 -> 1.5
+// forward, 6.2 -> 1.8 in a migration; 301 x 1203 5.8 -> 1.75, 6.5 -> 2.1; 600 x 2000 6.9 ->
+// 2.7, 7.6 -> 3.3; 1000 x 4000 11.2 -> 5.2, 13.4 -> 6.7 (600 Gpts/s).  Small grids are
+// bound by the chain edge -> packet -> neighbour's halo (about 1.4 us), large ones by
 // issue slots: some 110 instructions per four points, half of the slots used.  The
 // arithmetic is packed (.f32x2) for those slots; a packed instruction takes the pipe as
 // long as the two it replaces.

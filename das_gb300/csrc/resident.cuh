@@ -71,7 +71,8 @@ constexpr int RS_TILE_FLOATS = 64, RS_SHOT_FLOATS = 96;  // the tile's and the s
 __host__ __device__ inline size_t rs_smem_floats(int nrows, int ncol)
 {
     const size_t pitch = 4 * (size_t)ncol;
-    return RS_TILE_FLOATS + RS_SHOT_FLOATS + 2 * (nrows + 4) * pitch + 8 * (size_t)nrows + 4 * pitch + (nrows + 3) / 4 * 4 + 24;
+    return RS_TILE_FLOATS + RS_SHOT_FLOATS + 2 * (nrows + 4) * pitch + 8 * (size_t)nrows +
+           4 * pitch + (nrows + 3) / 4 * 4 + 24;
 }
 
 // Phase I of a tile: columns 1..ncol-2 by rows 2..nrows-3 in segments of R rows.
