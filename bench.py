@@ -477,7 +477,8 @@ def run_ours(args, dist):
                                              committed_traffic("cold_traffic_bytes_per_launch")),
                             "limiter": "issue slots: the wavefields and the model stay in "
                                        "shared and tensor memory for a whole pass, so DRAM "
-                                       "carries the snapshots alone (traffic: per step); frac is "
+                                       "carries the snapshots alone (traffic: per step, from a "
+                                       "pass without snapshots, which add 16 MB each); frac is "
                                        "the bytes a launch per step would move over the HBM "
                                        "copy rate" if on_chip else
                                        "latency: the three wave planes and the model (64 MB) "
