@@ -473,9 +473,16 @@ RsShot rs_shot(w2d_engine* e)
     return s;
 }
 
-// Phase steps [s.k0, s.k1) in one launch.
+// Phase steps [s.k0, s.k1) in one launch.  Never part of a captured pass: the launch holds the
+// shot's geometry and its tags by value, and a replay would use them for another shot.
 int rs_run(w2d_engine* e, RsShot& s)
 {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    W2D_CUDA_TRY(cudaStreamIsCapturing(e->stream, &cap));
+    if (cap != cudaStreamCaptureStatusNone) {
+        set_error("a resident launch does not go into a captured pass");
+        return W2D_ECUDA;
+    }
     // no packet of an earlier launch carries one of this launch's tags
     if (e->rs_tag > 0x70000000u) {
         W2D_CUDA_TRY(cudaMemsetAsync(e->rs_x.p, 0, e->rs.xbuf_bytes(), e->stream));
@@ -500,7 +507,8 @@ struct FwdOpts {
     int ckpt_every = 0;
 };
 
-int run_forward_steps(w2d_engine* e, int slot, const FwdOpts& o, int it0, int it1, double dt2inj,
+// on_chip: in the resident form (resident(), decided once by the caller for the whole pass).
+int run_forward_steps(w2d_engine* e, int slot, const FwdOpts& o, int it0, int it1, bool on_chip,
                       float dt2inj_f)
 {
     const AcGeom g = geom(e);
@@ -515,8 +523,6 @@ int run_forward_steps(w2d_engine* e, int slot, const FwdOpts& o, int it0, int it
             if (o.illum) s.illum = e->illum.p;
         }
     };
-    // (a recomputed segment samples no receivers, but they are on the device all the same)
-    const bool on_chip = resident(e, e->h_shot[3], true);
     for (int it = it0; it < it1;) {
         if (o.ckpt && o.ckpt_every > 0 && it % o.ckpt_every == 0) {
             e->chain = false;
@@ -569,7 +575,6 @@ int run_forward_steps(w2d_engine* e, int slot, const FwdOpts& o, int it0, int it
         }
         if (rc) return rc;
     }
-    (void)dt2inj;
     return W2D_OK;
 }
 
@@ -586,10 +591,10 @@ int forward_begin(w2d_engine* e, float dt2inj_f)
 }
 
 // Backward steps for it in [it_lo, it_hi] descending; m = nt-1-it picks roles
-// on the backward triple.  snaps: slot of step it = it/interval - slot0.
+// on the backward triple.  snaps: slot of step it = it/interval - slot0.  on_chip: as above.
 int run_backward_steps(w2d_engine* e, int slot, int nt, int interval, int n_rec, int it_hi,
                        int it_lo, const float* snaps, int slot0, int n_snaps_valid,
-                       float img_dt, float dt2inj_f)
+                       bool on_chip, float img_dt, float dt2inj_f)
 {
     const AcGeom g = geom(e);
     e->chain = false;  // the caller may have enqueued anything before these steps
@@ -606,7 +611,7 @@ int run_backward_steps(w2d_engine* e, int slot, int nt, int interval, int n_rec,
             }
         }
     };
-    if (resident(e, n_rec, false)) {
+    if (on_chip) {
         RsShot r = rs_shot(e);
         r.src_ix = -1;
         r.nt = nt;
@@ -679,8 +684,8 @@ std::vector<uintptr_t> pass_key(const w2d_engine* e, int pass, int nt, int inter
 // from `body` (the host code that launches it), instantiate and launch the graph.  With
 // graphs off, or in a launch mode that keeps host-side state, `body` runs directly.  A
 // capture the runtime refuses turns graphs off for this engine and runs `body`.
-// Nor a pass in the resident form: it is a launch or two as it is, by shot-specific
-// arguments.
+// Nor a pass with steps in the resident form (on_chip): those are a launch or two as they are,
+// by shot-specific arguments that no key holds.
 template <typename F>
 int run_pass(w2d_engine* e, w2d_engine::PassGraph& pg, std::vector<uintptr_t> key, bool on_chip,
              F&& body)
@@ -1033,6 +1038,7 @@ int w2d_forward(w2d_engine* e, int vel_slot, const float* wavelet, int nt, int s
     e->last_storage = 0;
     const float dt2inj = (float)(e->dt_d * e->dt_d);
     cudaEventRecord(e->ev0, e->stream);
+    const bool on_chip = resident(e, n_rec, true);
     auto pass = [&]() -> int {
         int r;
         if ((r = forward_begin(e, dt2inj))) return r;
@@ -1042,11 +1048,11 @@ int w2d_forward(w2d_engine* e, int vel_slot, const float* wavelet, int nt, int s
         o.n_rec = n_rec;
         o.rec_out = n_rec > 0 ? e->rec_out.p : nullptr;
         o.snaps = snaps_out ? e->snaps.p : nullptr;
-        return run_forward_steps(e, vel_slot, o, 0, nt, 0.0, dt2inj);
+        return run_forward_steps(e, vel_slot, o, 0, nt, on_chip, dt2inj);
     };
     const int kind = (vel_slot << 2) | (snaps_out ? 1 : 0) | (n_rec > 0 ? 2 : 0);
     if ((rc = run_pass(e, e->g_model, pass_key(e, 2, nt, snapshot_interval, kind, 0, n_rec),
-                       resident(e, n_rec, true), pass)))
+                       on_chip, pass)))
         return rc;
     cudaEventRecord(e->ev1, e->stream);
     if (n_rec > 0)
@@ -1103,6 +1109,7 @@ int w2d_backward_correlate(w2d_engine* e, int vel_slot, const float* data, int n
     const float dt2inj = (float)(e->dt_d * e->dt_d);
     const float img_dt = (float)(e->dt_d * (double)snapshot_interval);
     cudaEventRecord(e->ev0, e->stream);
+    const bool on_chip = resident(e, n_rec, false);
     auto pass = [&]() -> int {
         int r;
         if (n_rec > 0) {
@@ -1111,12 +1118,12 @@ int w2d_backward_correlate(w2d_engine* e, int vel_slot, const float* data, int n
             if ((r = zero_pass(e, 1))) return r;
         }
         return run_backward_steps(e, vel_slot, nt, snapshot_interval, n_rec, nt - 1, 0,
-                                  n_snaps > 0 ? e->snaps.p : nullptr, 0, n_snaps, img_dt,
+                                  n_snaps > 0 ? e->snaps.p : nullptr, 0, n_snaps, on_chip, img_dt,
                                   dt2inj);
     };
     if ((rc = run_pass(e, e->g_bcorr,
-                       pass_key(e, 3, nt, snapshot_interval, vel_slot, n_snaps, n_rec),
-                       resident(e, n_rec, false), pass)))
+                       pass_key(e, 3, nt, snapshot_interval, vel_slot, n_snaps, n_rec), on_chip,
+                       pass)))
         return rc;
     cudaEventRecord(e->ev1, e->stream);
     if ((rc = download_field(e, image, e->image.p))) return rc;
@@ -1175,6 +1182,10 @@ int migrate_core(w2d_engine* e, int nt, int n_rec, int snapshot_interval, int st
     const float img_dt = (float)(e->dt_d * (double)interval);
     cudaEventRecord(e->ev0, e->stream);
 
+    // The form of each pass's steps, decided here for the whole migration: the backward
+    // pass has no source and may run on chip where the forward one does not.
+    const bool fwd_chip = resident(e, n_rec, true), bwd_chip = resident(e, n_rec, false);
+
     // 1. forward pass in slot 0 with illumination
     auto forward = [&]() -> int {
         int r;
@@ -1191,14 +1202,14 @@ int migrate_core(w2d_engine* e, int nt, int n_rec, int snapshot_interval, int st
             o.ckpt = e->ckpt.p;
             o.ckpt_every = seg;
         }
-        if ((r = run_forward_steps(e, 0, o, 0, nt, 0.0, dt2inj))) return r;
+        if ((r = run_forward_steps(e, 0, o, 0, nt, fwd_chip, dt2inj))) return r;
         scale_kernel<<<grid_for(e->plane), 256, 0, e->stream>>>(e->illum.p, e->plane, img_dt);
         e->last_launches++;
         W2D_CUDA_TRY(cudaGetLastError());
         return W2D_OK;
     };
-    if ((rc = run_pass(e, e->g_fwd, pass_key(e, 0, nt, interval, mode, seg, n_rec),
-                       resident(e, n_rec, true), forward)))
+    if ((rc = run_pass(e, e->g_fwd, pass_key(e, 0, nt, interval, mode, seg, n_rec), fwd_chip,
+                       forward)))
         return rc;
     if (image_out) W2D_CUDA_TRY(cudaEventRecord(e->fwd_done, e->stream));
 
@@ -1216,7 +1227,7 @@ int migrate_core(w2d_engine* e, int nt, int n_rec, int snapshot_interval, int st
         }
         if (mode == W2D_STORE_ALL)
             return run_backward_steps(e, 1, nt, interval, n_rec, nt - 1, 0, e->snaps.p, 0,
-                                      n_snaps, img_dt, dt2inj);
+                                      n_snaps, bwd_chip, img_dt, dt2inj);
         for (int sgi = n_seg - 1; sgi >= 0; --sgi) {
             const int a = sgi * seg, b = std::min(nt, a + seg);
             // restore the forward state at step a and recompute [a, b) with snapshots
@@ -1233,17 +1244,17 @@ int migrate_core(w2d_engine* e, int nt, int n_rec, int snapshot_interval, int st
             r.snaps = e->snaps.p;
             r.slot0 = (a + interval - 1) / interval;  // first snapshot index in [a, b)
             int q;
-            if ((q = run_forward_steps(e, 0, r, a, b, 0.0, dt2inj))) return q;
+            if ((q = run_forward_steps(e, 0, r, a, b, fwd_chip, dt2inj))) return q;
             e->last_recompute += b - a;
             if ((q = run_backward_steps(e, 1, nt, interval, n_rec, b - 1, a, e->snaps.p, r.slot0,
-                                        n_snaps, img_dt, dt2inj)))
+                                        n_snaps, bwd_chip, img_dt, dt2inj)))
                 return q;
         }
         return W2D_OK;
     };
-    // (with checkpoints it recomputes forward segments: on chip as a whole or not at all)
-    if ((rc = run_pass(e, e->g_bwd, pass_key(e, 1, nt, interval, mode, seg, n_rec),
-                       resident(e, n_rec, mode != W2D_STORE_ALL), backward)))
+    // (captured only if it has no step on chip: where the forward steps are, so are these)
+    if ((rc = run_pass(e, e->g_bwd, pass_key(e, 1, nt, interval, mode, seg, n_rec), bwd_chip,
+                       backward)))
         return rc;
     cudaEventRecord(e->ev1, e->stream);
     if (image_out) {
@@ -1741,7 +1752,7 @@ int w2d_fwi_forward(w2d_engine* e, const float* vel_dev, const float* wavelet, i
         o.ckpt = e->ckpt.p;
         o.ckpt_every = f->seg;
     }
-    if ((rc = run_forward_steps(e, 0, o, 0, nt, 0.0, dt2inj))) return rc;
+    if ((rc = run_forward_steps(e, 0, o, 0, nt, resident(e, n_rec, true), dt2inj))) return rc;
     W2D_CUDA_TRY(cudaMemcpyAsync(traces_dev, e->rec_out.p, (size_t)nt * n_rec * 4,
                                  cudaMemcpyDeviceToDevice, e->stream));
     return check_err(e);
@@ -1800,7 +1811,7 @@ int w2d_fwi_gradient(w2d_engine* e, const float* resid_dev, float* grad_dev)
                 r.snaps = f->segbuf.p;
                 r.slot0 = a;
                 r.lap = true;
-                if ((rc = run_forward_steps(e, 0, r, a, b, 0.0, dt2inj))) return rc;
+                if ((rc = run_forward_steps(e, 0, r, a, b, true, dt2inj))) return rc;
                 e->last_recompute += b - a;
             }
             RsShot s = rs_shot(e);
@@ -1874,7 +1885,7 @@ int w2d_fwi_gradient(w2d_engine* e, const float* resid_dev, float* grad_dev)
             r.interval = 1;
             r.snaps = f->segbuf.p;
             r.slot0 = a;
-            if ((rc = run_forward_steps(e, 0, r, a, b, 0.0, dt2inj))) return rc;
+            if ((rc = run_forward_steps(e, 0, r, a, b, resident(e, n_rec, true), dt2inj))) return rc;
             e->last_recompute += b - a;
             adj_chain = false;  // the segment's first adjoint step waits for the stream
         }
