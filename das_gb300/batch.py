@@ -236,9 +236,14 @@ class BatchEngine:
         _lib.check(self._lib.w2d_batch_cancel(self._h, int(slot)))
 
     def fetch(self, slot: int, nz: int, nx: int, out=None) -> Tuple[np.ndarray, np.ndarray]:
-        """(image, illumination) of a finished migration, into the arrays ``out`` if given."""
+        """(image, illumination) of a finished migration, into the arrays ``out`` if given:
+        two writable C-contiguous float32 (nz, nx) arrays."""
         img, ill = out if out is not None else (np.empty((nz, nx), np.float32),
                                                 np.empty((nz, nx), np.float32))
+        for a in (img, ill):  # the copy back writes nz * nx floats from their first element on
+            if not (isinstance(a, np.ndarray) and a.dtype == np.float32 and a.shape == (nz, nx)
+                    and a.flags.c_contiguous and a.flags.writeable):
+                raise ValueError("out must be two writable C-contiguous float32 (nz, nx) arrays")
         _lib.check(self._lib.w2d_batch_fetch(self._h, int(slot), img.ctypes.data, ill.ctypes.data))
         return img, ill
 

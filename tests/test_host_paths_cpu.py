@@ -54,3 +54,41 @@ def test_no_resident_launch_is_captured(fake, storage, source, line):
         assert n["cooperative"] >= 4 and n["captures"] == 0
     if line != "all":
         assert n["cooperative"] == 0 and n["captures"] == 2 and n["graph"] == 4
+
+
+class _Fetched:
+    """The C entry that copies results back, as calls that reached it."""
+
+    def __init__(self):
+        self.calls = 0
+
+    def w2d_batch_fetch(self, *args):
+        self.calls += 1
+        return 0
+
+
+@pytest.mark.parametrize("make", [
+    lambda: np.empty((4, 6), np.float32),                    # smaller
+    lambda: np.empty((6, 5), np.float32),                    # transposed
+    lambda: np.empty((5, 6), np.float64),
+    lambda: np.empty((5, 6), np.float16),
+    lambda: np.empty((5, 12), np.float32)[:, ::2],           # strided
+    lambda: np.empty((6, 5), np.float32).T,                  # other order
+    lambda: np.empty(30, np.float32),                        # one dimension
+    lambda: np.broadcast_to(np.float32(0), (5, 6)),          # read-only
+    lambda: [[0.0] * 6] * 5,
+])
+@pytest.mark.parametrize("place", [0, 1])
+def test_fetch_refuses_arrays_that_the_copy_would_overrun(make, place):
+    from das_gb300.batch import BatchEngine
+    eng = object.__new__(BatchEngine)
+    eng._lib, eng._h = _Fetched(), None
+    ok = [np.empty((5, 6), np.float32), np.empty((5, 6), np.float32)]
+    out = list(ok)
+    out[place] = make()
+    with pytest.raises(ValueError):
+        eng.fetch(0, 5, 6, out)
+    assert eng._lib.calls == 0
+    got = eng.fetch(0, 5, 6, ok)
+    assert got[0] is ok[0] and got[1] is ok[1] and eng._lib.calls == 1
+    assert eng.fetch(0, 5, 6)[0].shape == (5, 6)
