@@ -805,9 +805,12 @@ int grow_table(w2d_batch* b, T** p, size_t* cap, size_t n)
     return W2D_OK;
 }
 
-// The waves' tables for a new active set.
-int upload_waves(w2d_batch* b)
+// The waves of a new active set and their tables.  Without memory for the tables (a few MB,
+// wanted when the user's arena may have taken what the device had) there are none, and the
+// step kernels run every shot.
+int plan_waves(w2d_batch* b)
 {
+    b->waves = make_waves(b);
     size_t n_items = 0, packets = 0;
     for (const Wave& w : b->waves) {
         size_t p = 0;
@@ -817,9 +820,12 @@ int upload_waves(w2d_batch* b)
     }
     if (n_items == 0) return W2D_OK;
     int rc;
-    if ((rc = grow_table(b, &b->d_rs_items, &b->rs_items_cap, n_items))) return rc;
     const size_t had = b->rs_x_cap;
-    if ((rc = grow_table(b, &b->d_rs_x, &b->rs_x_cap, packets))) return rc;
+    if ((rc = grow_table(b, &b->d_rs_items, &b->rs_items_cap, n_items)) ||
+        (rc = grow_table(b, &b->d_rs_x, &b->rs_x_cap, packets))) {
+        b->waves.clear();
+        return rc == W2D_ENOMEM ? W2D_OK : rc;
+    }
     if (b->rs_x_cap != had) {
         W2D_CUDA_TRY(cudaMemsetAsync(b->d_rs_x, 0, b->rs_x_cap * sizeof(uint4), b->st));
         b->rs_tag = 0;
@@ -912,11 +918,11 @@ int w2d_batch_launch(w2d_batch* b)
     int rc;
     if (b->active_dirty) {
         b->waves.clear();
-        if (b->form == 1) b->waves = make_waves(b);
-        // the shots that advance by step kernels (the queue form: every shot)
+        if (b->form == 1 && (rc = plan_waves(b))) return rc;
+        // the shots that advance by step kernels (without waves every shot)
         std::vector<int> stepped;
         for (int s : b->active)
-            if (b->form != 1 || b->hs[s].plans.empty()) stepped.push_back(s);
+            if (b->waves.empty() || b->hs[s].plans.empty()) stepped.push_back(s);
         b->n_step = (int)stepped.size();
         std::vector<int> prefix(b->active.size() + 1, 0);
         for (size_t i = 0; i < b->active.size(); ++i)
@@ -942,7 +948,6 @@ int w2d_batch_launch(w2d_batch* b)
             if (b->t_all)
                 W2D_CUDA_TRY(cudaMemcpyAsync(b->d_items, items.data(), items.size() * sizeof(int2),
                                              cudaMemcpyHostToDevice, b->st));
-            if ((rc = upload_waves(b))) return rc;
         }
         b->active_dirty = false;
     }

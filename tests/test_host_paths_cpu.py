@@ -92,3 +92,24 @@ def test_fetch_refuses_arrays_that_the_copy_would_overrun(make, place):
     got = eng.fetch(0, 5, 6, ok)
     assert got[0] is ok[0] and got[1] is ok[1] and eng._lib.calls == 1
     assert eng.fetch(0, 5, 6)[0].shape == (5, 6)
+
+
+def test_batch_without_memory_for_the_waves_runs_step_kernels(fake):
+    """The waves' packet table is wanted when jobs run, after the arena took its memory:
+    without it every shot advances by step kernels, and on chip again when there is room."""
+    from das_gb300.batch import BatchEngine, ShotJob
+    nz, nx, nt = 600, 2000, 40
+    v, w, d = _vel(nz, nx), np.zeros(nt, np.float32), np.zeros((nt, nx), np.float32)
+    jobs = [ShotJob(nx, nz, 5.0, 5.0, 5e-4, v, v, w, d, np.arange(nx), nx // 2, 2, 2, 2, 10,
+                    0.0015, True) for _ in range(3)]
+    eng = BatchEngine(arena_bytes=4 << 30, max_shots=8)
+    fake.fake_set_total(fake.fake_used() + (1 << 20))
+    fake_device.counts(fake)
+    res, _ = eng.run(jobs)
+    n = fake_device.counts(fake)
+    assert len(res) == 3 and n["cooperative"] == 0 and n["graph"] > 0 and n["captures"] > 0
+    fake.fake_set_total(288 << 30)
+    res, _ = eng.run(jobs)
+    n = fake_device.counts(fake)
+    assert len(res) == 3 and n["cooperative"] > 0 and n["captured_cooperative"] == 0
+    eng.close()
