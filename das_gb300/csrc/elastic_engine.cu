@@ -61,6 +61,7 @@ struct w2d_elastic {
     CUtensorMap map_state;                  // 3D map over the S x 5 planes of `state`
     CUtensorMap map_seg;                    // and over all slots of `seg`
     bool stored = false;                    // `seg` holds every forward state
+    bool keep_next = true;                  // the next forward call may keep them
     int adj_form = 1;                       // 1: TMA-tiled adjoint passes, 0: per-cell kernels
     // every shot of the next batch has the same model: its parameters are stored once and
     // read by every shot (parameter stride 0), so a tile's parameters come from L2 for
@@ -296,6 +297,8 @@ int w2d_elastic_forward_batch(w2d_elastic* e, int n_shots, const float* lam, con
         W2D_CHECK_ARG(rec_ix[k] >= 2 && rec_ix[k] < e->nx - 2, "receiver_ix must be in [2, nx-2)");
     int rc;
     const int S = n_shots;
+    const bool keep = e->keep_next;
+    e->keep_next = true;
     e->have_forward = false;
     e->S = S;
     e->nt = nt;
@@ -305,10 +308,12 @@ int w2d_elastic_forward_batch(w2d_elastic* e, int n_shots, const float* lam, con
     const size_t P = e->plane, SS = e->SS();
     // Every state kept where they all fit an eighth of the free memory (the rest stays for
     // others): nothing is recomputed (forward and gradient, 4 shots of 363 x 725, 700 steps:
-    // 41.6 -> 31.0 ms; 1024 x 2048, 500 steps: 52.5 -> 41.4).
+    // 41.6 -> 31.0 ms; 1024 x 2048, 500 steps: 52.5 -> 41.4).  Not where no gradient follows:
+    // a forward pass alone is faster in place, its state in L2 from step to step (the same
+    // two: 11.8 ms with the states kept and 11.4 without, 13.0 and 11.2).
     const size_t all = (size_t)(nt + 1) * S * SS;
     e->stored = false;
-    if ((size_t)(nt + 1) * S * 5 <= 0x7fffffff) {
+    if (keep && (size_t)(nt + 1) * S * 5 <= 0x7fffffff) {
         size_t fr = 0, tot = 0;
         if (all > e->seg_cap) cudaMemGetInfo(&fr, &tot);
         e->stored = (all <= e->seg_cap || all * 4 <= fr / 8) &&
@@ -399,6 +404,13 @@ int w2d_elastic_forward_batch(w2d_elastic* e, int n_shots, const float* lam, con
     if ((rc = check_el_err(e))) return rc;
     cudaEventElapsedTime(&e->last_ms, e->e0, e->e1);
     e->have_forward = true;
+    return W2D_OK;
+}
+
+int w2d_elastic_keep_states(w2d_elastic* e, int on)
+{
+    W2D_CHECK_ARG(e, "handle is NULL");
+    e->keep_next = on != 0;
     return W2D_OK;
 }
 

@@ -7,7 +7,8 @@ vertical-strain receivers -- the quantity a DAS fibre records -- and
 ``ElasticModeling`` puts the hand-written adjoint behind torch.autograd, so the
 gradient of any loss on the traces with respect to lambda, mu and the
 buoyancies (and, through ``gardner_parameters``, with respect to the shear
-velocity) is available, the forward states being recomputed from checkpoints.
+velocity) is available, over the forward states kept during the forward run where they
+fit an eighth of the free memory, and recomputed from checkpoints otherwise.
 """
 from __future__ import annotations
 
@@ -116,6 +117,8 @@ class ElasticModeling(torch.autograd.Function):
         shared = batched and S > 1 and solver.share_models and all(
             bool(torch.equal(t, t[:1].expand_as(t))) for t in ps)
         _lib.check(solver._lib.w2d_elastic_share_model(solver._h, 1 if shared else 0))
+        _lib.check(solver._lib.w2d_elastic_keep_states(
+            solver._h, 1 if any(ctx.needs_input_grad[:4]) else 0))
         torch.cuda.current_stream(ps[0].device).synchronize()
         _lib.check(solver._lib.w2d_elastic_forward_batch(
             solver._h, S, *[t.data_ptr() for t in ps], w.ctypes.data, nt, six.ctypes.data,

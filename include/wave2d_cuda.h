@@ -236,8 +236,8 @@ int w2d_elastic_forward(w2d_elastic* e, const float* lam, const float* mu, const
                         const float* bz, const float* wavelet, int nt, int src_ix, int src_iz,
                         const int* rec_ix, int n_rec, int rec_iz, float* traces_dev);
 /* Gradients of sum(resid * traces) with respect to lambda, mu, buo_x, buo_z (any
- * output may be NULL); exact adjoint of the discrete step, forward states
- * recomputed from checkpoints. */
+ * output may be NULL); exact adjoint of the discrete step, over the forward states that
+ * the forward call kept or, where it kept checkpoints alone, recomputed from them. */
 int w2d_elastic_gradient(w2d_elastic* e, const float* resid_dev, float* g_lam, float* g_mu,
                          float* g_bx, float* g_bz);
 float w2d_elastic_last_ms(w2d_elastic* e);
@@ -269,6 +269,10 @@ int w2d_elastic_set_pdl(w2d_elastic* e, int on);
  * reads them (their tiles then come from L2 for all but the first shot).  Gradients
  * stay per shot.  Applies to that one call. */
 int w2d_elastic_share_model(w2d_elastic* e, int on);
+/* Whether the next forward call may keep every forward state for its gradient (1, as without
+ * this call) or is to keep checkpoints alone (0: no gradient is expected, though one may
+ * follow).  Applies to that one call; results are identical. */
+int w2d_elastic_keep_states(w2d_elastic* e, int on);
 /* Device bytes one shot of a batch holds (checkpoints, one recomputed segment, fields). */
 unsigned long long w2d_elastic_shot_bytes(int nx, int nz, int nt, int n_rec);
 
