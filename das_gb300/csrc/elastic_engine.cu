@@ -62,6 +62,8 @@ struct w2d_elastic {
     CUtensorMap map_seg;                    // and over all slots of `seg`
     bool stored = false;                    // `seg` holds every forward state
     bool keep_next = true;                  // the next forward call may keep them
+    unsigned long long budget = 0;          // device bytes within which it may (0: the free
+                                            // memory decides)
     int adj_form = 1;                       // 1: TMA-tiled adjoint passes, 0: per-cell kernels
     // every shot of the next batch has the same model: its parameters are stored once and
     // read by every shot (parameter stride 0), so a tile's parameters come from L2 for
@@ -109,6 +111,13 @@ int grow(T** p, size_t n, size_t* cap)
     }
     *cap = n;
     return W2D_OK;
+}
+
+void drop(float** p, size_t* cap)
+{
+    if (*p) cudaFree(*p);
+    *p = nullptr;
+    *cap = 0;
 }
 
 ElGeom egeom(w2d_elastic* e)
@@ -193,6 +202,15 @@ bool on_m(const w2d_elastic* e, int iz, int ix)
     return iz >= (e->fs ? 1 : 2) && iz < e->nz - 2 && ix >= 2 && ix < e->nx - 2;
 }
 
+// Device bytes of one shot with `states` kept states (5 planes each): params 4, state 5, adj 5,
+// tmp 5, grad 4, the states, traces.
+size_t shot_bytes(int nx, int nz, int nt, int n_rec, size_t states)
+{
+    const size_t plane = (size_t)pitch_for(nx) * nz;
+    return (4 + 5 + 5 + 5 + 4 + states * 5) * plane * 4 + (size_t)nt * 4 +
+           (size_t)nt * std::max(n_rec, 1) * 4 + 64;
+}
+
 // checkpoint segments: about sqrt(3 nt) steps each
 void plan_segments(int nt, int* seg_len, int* n_seg)
 {
@@ -264,11 +282,8 @@ unsigned long long w2d_elastic_shot_bytes(int nx, int nz, int nt, int n_rec)
     if (nx < 5 || nz < 5 || nt <= 0) return 0;
     int seg_len = 0, n_seg = 0;
     plan_segments(nt, &seg_len, &n_seg);
-    const size_t plane = (size_t)pitch_for(nx) * nz;
-    // params 4, state 5, adj 5, tmp 5, grad 4, checkpoints, one segment of states
-    const size_t planes = 4 + 5 + 5 + 5 + 4 + (size_t)n_seg * 5 + (size_t)(seg_len + 1) * 5;
-    return (unsigned long long)(planes * plane * 4 + (size_t)nt * 4 +
-                                (size_t)nt * std::max(n_rec, 1) * 4 + 64);
+    // checkpoints and one segment of states
+    return shot_bytes(nx, nz, nt, n_rec, (size_t)n_seg + seg_len + 1);
 }
 
 // lam, mu, bx, bz: DEVICE arrays, n_shots x (nz, nx) contiguous.  wavelets: HOST
@@ -307,18 +322,23 @@ int w2d_elastic_forward_batch(w2d_elastic* e, int n_shots, const float* lam, con
     plan_segments(nt, &e->seg_len, &e->n_seg);
     const size_t P = e->plane, SS = e->SS();
     // Every state kept where they all fit an eighth of the free memory (the rest stays for
-    // others): nothing is recomputed (forward and gradient, 4 shots of 363 x 725, 700 steps:
+    // others), or the whole batch with them the budget: nothing is recomputed (forward and gradient, 4 shots of 363 x 725, 700 steps:
     // 41.6 -> 31.0 ms; 1024 x 2048, 500 steps: 52.5 -> 41.4).  Not where no gradient follows:
     // a forward pass alone is faster in place, its state in L2 from step to step (the same
     // two: 11.8 ms with the states kept and 11.4 without, 13.0 and 11.2).
     const size_t all = (size_t)(nt + 1) * S * SS;
-    e->stored = false;
-    if (keep && (size_t)(nt + 1) * S * 5 <= 0x7fffffff) {
+    bool fits = (size_t)(nt + 1) * S * 5 <= 0x7fffffff;
+    if (e->budget) {
+        fits &= S * shot_bytes(e->nx, e->nz, nt, n_rec, nt + 1) <= e->budget;
+    } else if (all > e->seg_cap) {
         size_t fr = 0, tot = 0;
-        if (all > e->seg_cap) cudaMemGetInfo(&fr, &tot);
-        e->stored = (all <= e->seg_cap || all * 4 <= fr / 8) &&
-                    grow(&e->seg, all, &e->seg_cap) == W2D_OK;
+        cudaMemGetInfo(&fr, &tot);
+        fits &= all * 4 <= fr / 8;
     }
+    // what a run before this one needed and this one does not goes back
+    if (!fits && e->seg_cap > (size_t)(e->seg_len + 1) * S * SS) drop(&e->seg, &e->seg_cap);
+    if (fits && keep && e->budget) drop(&e->ckpt, &e->ckpt_cap);
+    e->stored = fits && keep && grow(&e->seg, all, &e->seg_cap) == W2D_OK;
     if (e->stored) {
         e->seg_len = nt;
         e->n_seg = 1;
@@ -404,6 +424,19 @@ int w2d_elastic_forward_batch(w2d_elastic* e, int n_shots, const float* lam, con
     if ((rc = check_el_err(e))) return rc;
     cudaEventElapsedTime(&e->last_ms, e->e0, e->e1);
     e->have_forward = true;
+    return W2D_OK;
+}
+
+int w2d_elastic_set_memory_budget(w2d_elastic* e, unsigned long long bytes)
+{
+    W2D_ON_DEVICE_OF(e);
+    W2D_CHECK_ARG(e, "handle is NULL");
+    e->budget = bytes;
+    if (bytes && e->seg_cap * 4 > bytes) {
+        W2D_CUDA_TRY(cudaStreamSynchronize(e->st));
+        drop(&e->seg, &e->seg_cap);
+        e->have_forward = false;
+    }
     return W2D_OK;
 }
 

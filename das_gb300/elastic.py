@@ -58,6 +58,14 @@ class ElasticSolver2D:
         _lib.check(self._lib.w2d_elastic_set_tiles(self._h, int(step[0]), int(step[1]),
                                                    int(adjoint[0]), int(adjoint[1])))
 
+    def set_memory_budget(self, nbytes: int = 0):
+        """Device bytes within which a batch may keep every forward state for its gradient
+        (nothing is recomputed then); a batch that needs more keeps checkpoints.  0 (the
+        default): kept where the states fit an eighth of the free memory, in a buffer that
+        stays with the solver.  A kept buffer above the budget is freed at once (a gradient
+        then needs a new forward run).  Results are the same bit for bit."""
+        _lib.check(self._lib.w2d_elastic_set_memory_budget(self._h, int(nbytes)))
+
     def set_pdl(self, on: bool = True):
         """Programmatic dependent launches between consecutive step and tiled-adjoint
         kernels (on by default); results are identical either way."""
@@ -182,12 +190,18 @@ class ElasticExecutor:
     def _key(s):
         return (s.nx, s.nz, s.dx, s.dz, s.dt, s.n_sponge, s.sponge_alpha, s.free_surface_top)
 
+    def _make_solver(self, s):
+        """A solver for shot s that stays within the per-worker budget."""
+        solver = ElasticSolver2D(s.nx, s.nz, s.dx, s.dz, s.dt, s.n_sponge, s.sponge_alpha,
+                                 s.free_surface_top)
+        solver.set_memory_budget(self.budget)
+        return solver
+
     def _solver(self, s):
         """A solver for shot s kept by the calling thread's caller (used outside the workers)."""
         key = self._key(s)
         if key not in self._solvers:
-            self._solvers[key] = ElasticSolver2D(s.nx, s.nz, s.dx, s.dz, s.dt, s.n_sponge,
-                                                 s.sponge_alpha, s.free_surface_top)
+            self._solvers[key] = self._make_solver(s)
         return self._solvers[key]
 
     @staticmethod
@@ -254,9 +268,7 @@ class ElasticExecutor:
                 if solver is not None:
                     solver.close()
                 key = self._key(shots[0])
-                s0 = shots[0]
-                solver = ElasticSolver2D(s0.nx, s0.nz, s0.dx, s0.dz, s0.dt, s0.n_sponge,
-                                         s0.sponge_alpha, s0.free_surface_top)
+                solver = self._make_solver(shots[0])
             tb = time.perf_counter()
             res = self.migrate_shots(solver, shots)
             with self._lock:

@@ -269,11 +269,17 @@ int w2d_elastic_set_pdl(w2d_elastic* e, int on);
  * reads them (their tiles then come from L2 for all but the first shot).  Gradients
  * stay per shot.  Applies to that one call. */
 int w2d_elastic_share_model(w2d_elastic* e, int on);
+/* Bounds what a handle keeps for its gradients.  Without a budget (0) every forward state is
+ * kept where they fit an eighth of the free memory, in a buffer that stays with the handle
+ * until a run does not fit; with one they are kept only where all that the batch holds fits
+ * `bytes`, and else checkpoints are, whatever they take.  A kept buffer larger than `bytes`
+ * is freed by this call (a gradient then wants a new forward call). */
+int w2d_elastic_set_memory_budget(w2d_elastic* e, unsigned long long bytes);
 /* Whether the next forward call may keep every forward state for its gradient (1, as without
  * this call) or is to keep checkpoints alone (0: no gradient is expected, though one may
  * follow).  Applies to that one call; results are identical. */
 int w2d_elastic_keep_states(w2d_elastic* e, int on);
-/* Device bytes one shot of a batch holds (checkpoints, one recomputed segment, fields). */
+/* Device bytes one shot of a batch holds with checkpoints (and one recomputed segment, fields). */
 unsigned long long w2d_elastic_shot_bytes(int nx, int nz, int nt, int n_rec);
 
 /* ---- Part 3: batched / continuously fed migration (no reference counterpart:

@@ -30,7 +30,7 @@ def test_a_forward_run_without_gradient_keeps_no_states():
     import torch
     states = (NT + 1) * S * 5 * NZ * 288 * 4  # bytes, rows of 288 floats
     solver, vs, w = _setup()
-    _run(solver, vs[:, :, :], w[:4], False)  # what the first call loads and allocates
+    _run(solver, vs, w[:4], False)  # what the first call loads and allocates
     free0 = torch.cuda.mem_get_info()[0]
     tr0, _ = _run(solver, vs, w, False)
     free1 = torch.cuda.mem_get_info()[0]
@@ -44,3 +44,20 @@ def test_a_forward_run_without_gradient_keeps_no_states():
     for t in (tr1, tr2, tr3):
         np.testing.assert_array_equal(tr0, t)
     np.testing.assert_array_equal(g1, g3)
+
+
+def test_results_do_not_depend_on_the_budget():
+    """States kept, kept again after they were given up, and checkpoints: the same traces and
+    gradients, also over runs of other lengths and batches on one solver."""
+    solver, vs, w = _setup()
+    ref = _run(solver, vs, w, True)
+    short = _run(solver, vs[:1].repeat(2, 1, 1), w[:90], True)
+    for budget in (1 << 20, 1 << 33, 0, 1 << 20, 0):
+        solver.set_memory_budget(budget)
+        got = _run(solver, vs, w, True)
+        np.testing.assert_array_equal(got[0], ref[0])
+        np.testing.assert_array_equal(got[1], ref[1])
+        got = _run(solver, vs[:1].repeat(2, 1, 1), w[:90], True)
+        np.testing.assert_array_equal(got[0], short[0])
+        np.testing.assert_array_equal(got[1], short[1])
+    solver.close()

@@ -113,3 +113,58 @@ def test_batch_without_memory_for_the_waves_runs_step_kernels(fake):
     n = fake_device.counts(fake)
     assert len(res) == 3 and n["cooperative"] > 0 and n["captured_cooperative"] == 0
     eng.close()
+
+
+def _elastic_forward(lib, h, nz, nx, nt, n_shots):
+    """One forward call on stand-in device arrays."""
+    p = np.zeros(1, np.float32)
+    w = np.zeros((n_shots, nt), np.float32)
+    six, siz = np.full(n_shots, nx // 2, np.int32), np.full(n_shots, 2, np.int32)
+    rix = np.arange(2, nx - 2, dtype=np.int32)
+    return lib.w2d_elastic_forward_batch(h, n_shots, *[p.ctypes.data] * 4, w.ctypes.data, nt,
+                                         six.ctypes.data, siz.ctypes.data, rix.ctypes.data,
+                                         len(rix), 4, p.ctypes.data)
+
+
+def test_elastic_executor_stays_within_its_budget(fake):
+    """A worker's solver holds no more than the budget its batches are sized by, over batches
+    of one to four shots and of several lengths, whatever memory is free."""
+    from types import SimpleNamespace
+    from das_gb300.elastic import ElasticExecutor
+    nz, nx = 363, 725
+    ex = object.__new__(ElasticExecutor)
+    ex.budget, ex._solvers = 2 << 30, {}
+    s = ex._solver(SimpleNamespace(nx=nx, nz=nz, dx=5.0, dz=5.0, dt=5e-4, n_sponge=30,
+                                   sponge_alpha=0.0015, free_surface_top=True))
+    base = fake.fake_used()
+    for n_shots, nt in [(1, 100), (4, 700), (1, 250), (1, 3000), (2, 100), (4, 700), (1, 100)]:
+        per = fake.w2d_elastic_shot_bytes(nx, nz, nt, nx - 4)
+        assert n_shots * per <= ex.budget
+        fake_device.counts(fake)
+        assert _elastic_forward(fake, s._h, nz, nx, nt, n_shots) == 0
+        # (tables of columns and checkpoints of other lengths beside it)
+        assert fake.fake_used() - base <= ex.budget + (600 << 20), (n_shots, nt)
+    s.close()
+
+
+def test_elastic_states_go_back(fake):
+    """Kept states are bounded and given back: by a budget below them, by a run whose states
+    do not fit, and with the solver."""
+    from das_gb300.elastic import ElasticSolver2D
+    nz, nx, nt = 363, 725, 700
+    states = (nt + 1) * 5 * nz * 736 * 4
+    start = fake.fake_used()
+    s = ElasticSolver2D(nx, nz, 5.0, 5.0, 5e-4)
+    assert _elastic_forward(fake, s._h, nz, nx, nt, 1) == 0
+    assert fake.fake_used() - start > states
+    s.set_memory_budget(1 << 30)
+    assert fake.fake_used() - start < states // 8
+    assert _elastic_forward(fake, s._h, nz, nx, nt, 1) == 0
+    assert fake.fake_used() - start <= 1 << 30
+    s.set_memory_budget(0)
+    assert _elastic_forward(fake, s._h, nz, nx, nt, 1) == 0
+    assert fake.fake_used() - start > states
+    assert _elastic_forward(fake, s._h, nz, nx, 20000, 1) == 0  # 107 GB of states
+    assert fake.fake_used() - start < states
+    s.close()
+    assert fake.fake_used() == start
