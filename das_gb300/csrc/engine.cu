@@ -212,6 +212,10 @@ struct w2d_engine {
     const CUtensorMap& mprev(int i) const { return map_prev[perm[i]]; }
 };
 
+// Bytes of the forward states that the gradient path keeps by its own choice, and giving them
+// back (false: there are none).
+static size_t fwi_kept(const w2d_fwi_state* f);
+static bool fwi_give_back(w2d_engine* e);
 static void fwi_free(w2d_fwi_state* f);
 
 namespace {
@@ -763,7 +767,15 @@ size_t free_budget(w2d_engine* e)
     if (e->budget) return (size_t)e->budget;
     size_t fr = 0, tot = 0;
     cudaMemGetInfo(&fr, &tot);
-    return (size_t)(fr * 0.8);
+    return (size_t)((fr + fwi_kept(e->fwi)) * 0.8);
+}
+
+// Snapshot and checkpoint storage, for which kept states make room.
+int ensure_storage(w2d_engine* e, DevBuf<float>& b, size_t n)
+{
+    int rc = b.ensure(n);
+    if (rc == W2D_ENOMEM && fwi_give_back(e)) rc = b.ensure(n);
+    return rc;
 }
 
 }  // namespace
@@ -987,6 +999,7 @@ int w2d_engine_set_memory_budget(w2d_engine* e, unsigned long long bytes)
     W2D_ON_DEVICE_OF(e);
     W2D_CHECK_ARG(e, "engine is NULL");
     e->budget = bytes;
+    if (bytes && fwi_kept(e->fwi) > bytes / 8) fwi_give_back(e);
     return W2D_OK;
 }
 
@@ -1028,7 +1041,7 @@ int w2d_forward(w2d_engine* e, int vel_slot, const float* wavelet, int nt, int s
             set_error("snapshot storage exceeds the device memory budget");
             return W2D_ENOMEM;
         }
-        if ((rc = e->snaps.ensure(need))) return rc;
+        if ((rc = ensure_storage(e, e->snaps, need))) return rc;
     }
     W2D_CUDA_TRY(cudaMemcpyAsync(e->wavelet.p, wavelet, (size_t)nt * 4, cudaMemcpyHostToDevice,
                                  e->stream));
@@ -1094,7 +1107,7 @@ int w2d_backward_correlate(w2d_engine* e, int vel_slot, const float* data, int n
             set_error("forward wavefields exceed the device memory budget");
             return W2D_ENOMEM;
         }
-        if ((rc = e->snaps.ensure(need))) return rc;
+        if ((rc = ensure_storage(e, e->snaps, need))) return rc;
         W2D_CUDA_TRY(cudaMemsetAsync(e->snaps.p, 0, need * 4, e->stream));
         for (int k = 0; k < n_snaps; ++k)
             if ((rc = upload_field(e, e->snaps.p + (size_t)k * e->plane,
@@ -1158,7 +1171,7 @@ int migrate_core(w2d_engine* e, int nt, int n_rec, int snapshot_interval, int st
             set_error("full snapshot storage exceeds the device memory budget");
             return W2D_ENOMEM;
         }
-        if ((rc = e->snaps.ensure((size_t)n_snaps * e->plane))) return rc;
+        if ((rc = ensure_storage(e, e->snaps, (size_t)n_snaps * e->plane))) return rc;
     } else {
         // segment length: about sqrt(3 * nt * interval) steps, rounded to the interval,
         // balancing 3-plane checkpoints against the snapshots of one segment.
@@ -1171,8 +1184,8 @@ int migrate_core(w2d_engine* e, int nt, int n_rec, int snapshot_interval, int st
             set_error("checkpoint storage exceeds the device memory budget");
             return W2D_ENOMEM;
         }
-        if ((rc = e->ckpt.ensure((size_t)n_seg * 3 * e->plane)) ||
-            (rc = e->snaps.ensure((size_t)seg_snaps * e->plane)))
+        if ((rc = ensure_storage(e, e->ckpt, (size_t)n_seg * 3 * e->plane)) ||
+            (rc = ensure_storage(e, e->snaps, (size_t)seg_snaps * e->plane)))
             return rc;
     }
     e->last_launches = 0;
@@ -1672,10 +1685,25 @@ struct w2d_fwi_state {
     int nt = 0, n_rec = 0, seg = 0, n_seg = 0;
     bool stored = false;  // one segment of every forward state, written by the forward pass
     bool lap = false;     // ... as its Laplacian, for the gradient in the resident form
+    bool all = false;     // ... because they fit, not because the caller asked for it
     DevBuf<float> vel_p, grad_c, zero, segbuf;
     std::vector<CUtensorMap> seg_maps;
     CUtensorMap map_c_halo, map_zero;
 };
+
+static size_t fwi_kept(const w2d_fwi_state* f)
+{
+    return f && f->all ? f->segbuf.cap * sizeof(float) : 0;
+}
+
+// (a gradient asked for afterwards runs its forward pass again, with checkpoints)
+static bool fwi_give_back(w2d_engine* e)
+{
+    if (!fwi_kept(e->fwi)) return false;
+    cudaStreamSynchronize(e->stream);
+    e->fwi->segbuf.release();
+    return true;
+}
 
 static void fwi_free(w2d_fwi_state* f)
 {
@@ -1683,6 +1711,60 @@ static void fwi_free(w2d_fwi_state* f)
     for (DevBuf<float>* b : {&f->vel_p, &f->grad_c, &f->zero, &f->segbuf}) b->release();
     delete f;
 }
+
+namespace {
+
+// How the forward states of the gradient path are kept, and the memory for it: all of them
+// (keep_all) where they fit an eighth of the memory at hand (the rest stays free for others)
+// and nothing is recomputed, else checkpoints.  Forward and gradient, 1000 x 4000, 600 steps:
+// 19.4 -> 13.5 ms, with fewer launches and the state's loads in fives.
+int fwi_plan(w2d_engine* e, w2d_fwi_state* f, bool keep_all)
+{
+    int rc;
+    const int nt = f->nt;
+    f->seg = e->fwi_seg > 0 ? std::min(e->fwi_seg, nt) : std::max(1, (int)std::sqrt(3.0 * nt));
+    const size_t all = (size_t)nt * e->plane;
+    const size_t room = e->budget ? (size_t)e->budget / 8
+                                  : std::max(free_budget(e) / 8, f->segbuf.cap * 4);
+    const bool keep = keep_all && e->fwi_seg <= 0 && fwi_resident(e, f->n_rec) &&
+                      all * 4 <= room && f->segbuf.ensure(all) == W2D_OK;
+    // what a run before this one kept and this one does not goes back
+    if (!keep && fwi_kept(f)) f->segbuf.release();
+    f->all = keep;
+    if (keep) f->seg = nt;
+    f->n_seg = (nt + f->seg - 1) / f->seg;
+    f->stored = f->seg >= nt;
+    f->lap = f->stored && fwi_resident(e, f->n_rec);
+    if ((rc = f->segbuf.ensure((size_t)f->seg * e->plane)) ||
+        (rc = e->ckpt.ensure((size_t)f->n_seg * 3 * e->plane)))
+        return rc;
+    return W2D_OK;
+}
+
+// The forward pass as planned, its receivers sampled into rec_out if given.
+int fwi_run_forward(w2d_engine* e, w2d_fwi_state* f, float* rec_out)
+{
+    const float dt2inj = (float)(e->dt_d * e->dt_d);
+    int rc;
+    if ((rc = forward_begin(e, dt2inj))) return rc;
+    FwdOpts o;
+    o.nt = f->nt;
+    o.n_rec = f->n_rec;
+    o.rec_out = rec_out;
+    if (f->stored) {
+        o.lap = f->lap;
+        // every forward state kept as it is computed: the gradient recomputes nothing
+        o.snaps = f->segbuf.p;
+        o.interval = 1;
+        o.slot0 = 0;
+    } else {
+        o.ckpt = e->ckpt.p;
+        o.ckpt_every = f->seg;
+    }
+    return run_forward_steps(e, 0, o, 0, f->nt, resident(e, f->n_rec, true), dt2inj);
+}
+
+}  // namespace
 
 extern "C" {
 
@@ -1709,19 +1791,9 @@ int w2d_fwi_forward(w2d_engine* e, const float* vel_dev, const float* wavelet, i
     if ((rc = set_shot(e, src_ix, src_iz, rec_ix, n_rec, rec_iz))) return rc;
     f->nt = nt;
     f->n_rec = n_rec;
-    f->seg = e->fwi_seg > 0 ? std::min(e->fwi_seg, nt) : std::max(1, (int)std::sqrt(3.0 * nt));
-    // Every state kept where they all fit an eighth of the memory at hand (the rest stays
-    // free for others): nothing is recomputed.  Forward and gradient, 1000 x 4000, 600
-    // steps: 19.4 -> 13.5 ms, with fewer launches and the state's loads in fives.
-    const size_t all = (size_t)nt * e->plane;
-    if (e->fwi_seg <= 0 && fwi_resident(e, n_rec) &&
-        all * 4 <= std::max(free_budget(e) / 8, f->segbuf.cap * 4) &&
-        f->segbuf.ensure(all) == W2D_OK)
-        f->seg = nt;
-    f->n_seg = (nt + f->seg - 1) / f->seg;
-    if ((rc = f->vel_p.ensure(e->plane)) || (rc = f->grad_c.ensure(e->plane)) ||
-        (rc = f->zero.ensure(e->plane)) || (rc = f->segbuf.ensure((size_t)f->seg * e->plane)) ||
-        (rc = e->ckpt.ensure((size_t)f->n_seg * 3 * e->plane)) || (rc = e->wavelet.ensure(nt)) ||
+    if ((rc = fwi_plan(e, f, true)) || (rc = f->vel_p.ensure(e->plane)) ||
+        (rc = f->grad_c.ensure(e->plane)) || (rc = f->zero.ensure(e->plane)) ||
+        (rc = e->wavelet.ensure(nt)) ||
         (rc = e->rec_out.ensure((size_t)nt * n_rec)) || (rc = e->data.ensure((size_t)nt * n_rec)))
         return rc;
     W2D_CUDA_TRY(cudaMemsetAsync(f->zero.p, 0, e->plane * 4, e->stream));
@@ -1734,25 +1806,7 @@ int w2d_fwi_forward(w2d_engine* e, const float* vel_dev, const float* wavelet, i
     e->cur_w = e->wavelet.p;
     e->last_launches = 0;
     e->last_recompute = 0;
-    const float dt2inj = (float)(e->dt_d * e->dt_d);
-    if ((rc = forward_begin(e, dt2inj))) return rc;
-    FwdOpts o;
-    o.nt = nt;
-    o.n_rec = n_rec;
-    o.rec_out = e->rec_out.p;
-    f->stored = f->seg >= nt;
-    f->lap = f->stored && fwi_resident(e, n_rec);
-    if (f->stored) {
-        o.lap = f->lap;
-        // every forward state kept as it is computed: the gradient recomputes nothing
-        o.snaps = f->segbuf.p;
-        o.interval = 1;
-        o.slot0 = 0;
-    } else {
-        o.ckpt = e->ckpt.p;
-        o.ckpt_every = f->seg;
-    }
-    if ((rc = run_forward_steps(e, 0, o, 0, nt, resident(e, n_rec, true), dt2inj))) return rc;
+    if ((rc = fwi_run_forward(e, f, e->rec_out.p))) return rc;
     W2D_CUDA_TRY(cudaMemcpyAsync(traces_dev, e->rec_out.p, (size_t)nt * n_rec * 4,
                                  cudaMemcpyDeviceToDevice, e->stream));
     return check_err(e);
@@ -1781,9 +1835,13 @@ int w2d_fwi_gradient(w2d_engine* e, const float* resid_dev, float* grad_dev)
     W2D_CHECK_DEVICE_PTR(resid_dev, e->device);
     W2D_CHECK_DEVICE_PTR(grad_dev, e->device);
     w2d_fwi_state* f = e->fwi;
+    int rc;
+    // the states were given back: once more, with checkpoints
+    if (f->all && !f->segbuf.p &&
+        ((rc = fwi_plan(e, f, false)) || (rc = fwi_run_forward(e, f, nullptr))))
+        return rc;
     const int nt = f->nt, n_rec = f->n_rec, seg = f->seg;
     const size_t plane_b = e->plane * 4;
-    int rc;
     W2D_CUDA_TRY(cudaMemcpyAsync(e->data.p, resid_dev, (size_t)nt * n_rec * 4,
                                  cudaMemcpyDeviceToDevice, e->stream));
     if ((rc = zero_pass(e, 1))) return rc;

@@ -138,8 +138,10 @@ class WaveSolver2D:
 
     def set_checkpoint_segment(self, steps: int = 0) -> None:
         """Steps per checkpoint segment of the differentiable path (das_gb300.autograd):
-        0 picks sqrt(3 nt); nt or more stores every forward state (no recomputation).
-        The gradient is the same bit for bit either way."""
+        nt or more stores every forward state (no recomputation); 0 stores them where the
+        grid runs on chip and they fit an eighth of the memory at hand (the engine keeps
+        that buffer until ``close()``, or until a migration's snapshots want the room), and
+        else picks sqrt(3 nt).  The gradient is the same bit for bit either way."""
         _lib.check(self._lib.w2d_fwi_set_segment(self._eng(), int(steps)))
 
     def set_adjoint_form(self, form: str = "tiled") -> None:

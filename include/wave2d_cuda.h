@@ -352,7 +352,10 @@ int w2d_batch_stats(w2d_batch* b, int* n_active, float* last_ms, double* last_po
                     long long* last_launches);
 
 /* Bytes of device memory the engine may use for snapshots/checkpoints (0 = 80 %
- * of free memory at the time of the call). */
+ * of free memory at the time of the call).  w2d_fwi_forward keeps every forward state for
+ * its gradient where they fit an eighth of that, in a buffer that stays with the engine;
+ * it makes room for a migration's snapshots, and a budget that it does not fit frees it
+ * (a gradient asked for afterwards recomputes its states). */
 int w2d_engine_set_memory_budget(w2d_engine* e, unsigned long long bytes);
 
 /* Statistics of the last whole-loop call: storage mode used (1 all, 2 checkpoint),

@@ -65,3 +65,30 @@ def test_modelling_and_correlation_of_changing_lines(source):
         for a, b in zip(*res):
             np.testing.assert_array_equal(a, b, err_msg=f"call {k}")
     kept.close()
+
+
+def test_gradient_after_its_states_were_given_back():
+    """The states kept for a gradient, given back before it (a budget below them), and a second
+    gradient of one forward run: the same bit for bit."""
+    import torch
+    from das_gb300.autograd import model_traces
+    from das_gb300.wave_solver import WaveSolver2D
+    nt = 200
+    rng = np.random.default_rng(8)
+    v = rng.uniform(1500, 3000, (NZ, NX)).astype(np.float32)
+    w = rng.standard_normal(nt).astype(np.float32)
+    rix = np.arange(2, NX - 2, 2)
+    r = torch.tensor(rng.standard_normal((nt, len(rix))).astype(np.float32), device="cuda")
+    s = WaveSolver2D(NX, NZ, 5.0, 5.0, 5e-4, n_sponge=12)
+    grads = []
+    for give_back in (False, True):
+        vt = torch.tensor(v, device="cuda", requires_grad=True)
+        d = model_traces(vt, s, w, NX // 3, 2, rix, 2)
+        if give_back:
+            assert s._lib.w2d_engine_set_memory_budget(s._eng(), 8 << 20) == 0
+        for _ in range(2):
+            grads.append(torch.autograd.grad(d, vt, r, retain_graph=True)[0].cpu().numpy())
+    s.close()
+    assert np.abs(grads[0]).max() > 0
+    for g in grads[1:]:
+        np.testing.assert_array_equal(grads[0], g)

@@ -168,3 +168,55 @@ def test_elastic_states_go_back(fake):
     assert fake.fake_used() - start < states
     s.close()
     assert fake.fake_used() == start
+
+
+def _fwi_forward(lib, solver, nt, n_rec=4):
+    """One forward call of the gradient path on stand-in device arrays."""
+    p, w = np.zeros(1, np.float32), np.zeros(nt, np.float32)
+    rix = np.arange(2, 2 + n_rec, dtype=np.int32)
+    return lib.w2d_fwi_forward(solver._eng(), p.ctypes.data, w.ctypes.data, nt, solver.nx // 2, 2,
+                               rix.ctypes.data, n_rec, 2, p.ctypes.data)
+
+
+def test_kept_states_make_room_for_snapshots(fake):
+    """The forward states that the gradient path keeps by its own choice do not count against
+    a migration's snapshots on the same engine: what fits an engine without them still runs,
+    and a gradient asked for afterwards recomputes its states."""
+    from das_gb300.rtm_engine import TSWRTMEngine
+    from das_gb300.velocity_flood import FloodModels
+    from das_gb300.wave_solver import WaveSolver2D
+    nz, nx, nt = 1000, 4000, 1500
+    s = WaveSolver2D(nx, nz, 5.0, 5.0, 5e-4)
+    v = _vel(nz, nx)
+    s.forward_propagate_acoustic(v, np.zeros(10, np.float32), nx // 2, 2, np.arange(4), 2)
+    base = fake.fake_used()
+    assert _fwi_forward(fake, s, nt) == 0
+    assert fake.fake_used() - base > nt * nz * nx * 4  # 24 GB
+    n = 13800  # 221 GB of snapshots: 80 % of the memory beside the states is 211 GB, of all 230
+    w, d = np.zeros(n, np.float32), np.zeros((n, 4), np.float32)
+    for storage in ("all", "auto"):
+        TSWRTMEngine(s, storage).migrate_shot(FloodModels(v, v, v, 0, 0), w, nx // 2, 2, d,
+                                              np.arange(4), 2, 1)
+        assert s.last_stats()["storage"] == "all"
+    s.close()
+
+    # and a gradient after the states were given back
+    assert _fwi_forward(fake, s, nt) == 0
+    kept = fake.fake_used()
+    _lib_check(fake, fake.w2d_engine_set_memory_budget(s._eng(), 1 << 30))
+    assert kept - fake.fake_used() >= nt * nz * nx * 4
+    p = np.zeros(1, np.float32)
+    fake_device.counts(fake)
+    _lib_check(fake, fake.w2d_fwi_gradient(s._eng(), p.ctypes.data, p.ctypes.data))
+    assert fake_device.counts(fake)["cooperative"] > 2
+    assert fake.fake_used() - base < nt * nz * nx * 4 // 2
+    # the budget bounds the next forward call too, and a run that does not fit keeps none
+    assert _fwi_forward(fake, s, nt) == 0 and fake.fake_used() - base < nt * nz * nx * 4 // 2
+    _lib_check(fake, fake.w2d_engine_set_memory_budget(s._eng(), 0))
+    assert _fwi_forward(fake, s, nt) == 0 and fake.fake_used() - base > nt * nz * nx * 4
+    assert _fwi_forward(fake, s, 8000) == 0 and fake.fake_used() - base < nt * nz * nx * 4 // 2
+    s.close()
+
+
+def _lib_check(lib, rc):
+    assert rc == 0, lib.w2d_last_error()
