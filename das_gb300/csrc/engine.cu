@@ -149,6 +149,7 @@ struct w2d_engine {
     DevBuf<int> shot;  // {src_ix, src_iz, rec_iz, n_rec, rec_c0}
     int h_shot[5] = {-1, -1, -1, 0, -1};  // host copy of the same
     bool one_per_column = true;           // no column holds two receivers
+    unsigned long long calls = 0;         // changes of the shot or of a model so far
 
     // resident form (resident.cu): how the grid is cut into tiles that stay on
     // chip (no plan where it does not fit), and the packets its tiles exchange
@@ -416,6 +417,7 @@ int set_shot(w2d_engine* e, int src_ix, int src_iz, const int* rec_ix, int n_rec
         return rc;
     int sh[5] = {src_ix, src_iz, rec_iz, n_rec, receivers_consecutive_c0(rec_ix, n_rec)};
     std::copy(sh, sh + 5, e->h_shot);
+    e->calls++;
     e->one_per_column = true;
     for (int i = 0; i < e->nx; ++i) e->one_per_column &= ptr[i + 1] - ptr[i] <= 1;
     W2D_CUDA_TRY(cudaMemcpyAsync(e->rec_ptr.p, ptr.data(), ptr.size() * 4, cudaMemcpyHostToDevice,
@@ -1009,6 +1011,7 @@ int w2d_engine_set_velocity(w2d_engine* e, int slot, const float* vel)
     W2D_CHECK_ARG(e && vel, "NULL argument");
     W2D_CHECK_ARG(slot == 0 || slot == 1, "velocity slot must be 0 or 1");
     int rc;
+    e->calls++;
     W2D_CUDA_TRY(cudaMemsetAsync(e->staging.p, 0, e->plane * 4, e->stream));
     if ((rc = upload_field_any(e, e->staging.p, vel))) return rc;
     v2dt2_kernel<<<grid_for(e->plane), 256, 0, e->stream>>>(e->v2dt2.p + (size_t)slot * e->plane,
@@ -1686,6 +1689,11 @@ struct w2d_fwi_state {
     bool stored = false;  // one segment of every forward state, written by the forward pass
     bool lap = false;     // ... as its Laplacian, for the gradient in the resident form
     bool all = false;     // ... because they fit, not because the caller asked for it
+    // the shot, for a gradient that other calls on the engine came before
+    int src_ix = 0, src_iz = 0, rec_iz = 0;
+    std::vector<int> rec_ix;
+    std::vector<float> wavelet;
+    unsigned long long calls = 0;  // the engine's count when its shot and model were this one's
     DevBuf<float> vel_p, grad_c, zero, segbuf;
     std::vector<CUtensorMap> seg_maps;
     CUtensorMap map_c_halo, map_zero;
@@ -1791,6 +1799,12 @@ int w2d_fwi_forward(w2d_engine* e, const float* vel_dev, const float* wavelet, i
     if ((rc = set_shot(e, src_ix, src_iz, rec_ix, n_rec, rec_iz))) return rc;
     f->nt = nt;
     f->n_rec = n_rec;
+    f->src_ix = src_ix;
+    f->src_iz = src_iz;
+    f->rec_iz = rec_iz;
+    f->rec_ix.assign(rec_ix, rec_ix + n_rec);
+    f->wavelet.assign(wavelet, wavelet + nt);
+    f->calls = e->calls;
     if ((rc = fwi_plan(e, f, true)) || (rc = f->vel_p.ensure(e->plane)) ||
         (rc = f->grad_c.ensure(e->plane)) || (rc = f->zero.ensure(e->plane)) ||
         (rc = e->wavelet.ensure(nt)) ||
@@ -1836,9 +1850,24 @@ int w2d_fwi_gradient(w2d_engine* e, const float* resid_dev, float* grad_dev)
     W2D_CHECK_DEVICE_PTR(grad_dev, e->device);
     w2d_fwi_state* f = e->fwi;
     int rc;
-    // the states were given back: once more, with checkpoints
-    if (f->all && !f->segbuf.p &&
-        ((rc = fwi_plan(e, f, false)) || (rc = fwi_run_forward(e, f, nullptr))))
+    bool again = f->all && !f->segbuf.p;  // the states were given back
+    if (f->calls != e->calls) {
+        // Other calls came between: this run's shot, wavelet and model once more (the kernels
+        // index the residuals by the engine's receivers).  The engine's checkpoints may be
+        // another pass's.
+        if ((rc = set_shot(e, f->src_ix, f->src_iz, f->rec_ix.data(), f->n_rec, f->rec_iz)) ||
+            (rc = e->wavelet.ensure(f->nt)))
+            return rc;
+        W2D_CUDA_TRY(cudaMemcpyAsync(e->wavelet.p, f->wavelet.data(), (size_t)f->nt * 4,
+                                     cudaMemcpyHostToDevice, e->stream));
+        e->cur_w = e->wavelet.p;
+        v2dt2_kernel<<<grid_for(e->plane), 256, 0, e->stream>>>(e->v2dt2.p, f->vel_p.p, e->plane,
+                                                                e->dt2);
+        W2D_CUDA_TRY(cudaGetLastError());
+        f->calls = e->calls;
+        again |= !f->stored;
+    }
+    if (again && ((rc = fwi_plan(e, f, false)) || (rc = fwi_run_forward(e, f, nullptr))))
         return rc;
     const int nt = f->nt, n_rec = f->n_rec, seg = f->seg;
     const size_t plane_b = e->plane * 4;

@@ -18,6 +18,7 @@ size_t total = (size_t)288 << 30, used = 0;
 bool capturing = false;
 // launches: plain, cooperative, cooperative inside a capture, graph; captures begun
 long long counts[5];
+char last[256];  // the first bytes of the last cooperative launch's first argument
 char handles[4096];
 unsigned next_handle = 0;
 
@@ -111,11 +112,14 @@ cudaError_t cudaGraphExecDestroy(cudaGraphExec_t) { return cudaSuccess; }
 cudaError_t cudaGraphDestroy(cudaGraph_t) { return cudaSuccess; }
 cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) { ++counts[3]; return cudaSuccess; }
 
-cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void*, void**)
+void fake_last_cooperative(void* out, int n) { memcpy(out, last, n); }
+
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void*, void** args)
 {
     for (unsigned i = 0; i < c->numAttrs; ++i)
         if (c->attrs[i].id == cudaLaunchAttributeCooperative && c->attrs[i].val.cooperative) {
             ++counts[capturing ? 2 : 1];
+            memcpy(last, args[0], sizeof last);
             return cudaSuccess;
         }
     ++counts[0];

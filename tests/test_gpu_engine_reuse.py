@@ -92,3 +92,40 @@ def test_gradient_after_its_states_were_given_back():
     assert np.abs(grads[0]).max() > 0
     for g in grads[1:]:
         np.testing.assert_array_equal(grads[0], g)
+
+
+@pytest.mark.parametrize("pdl", [True, False])
+@pytest.mark.parametrize("segment", [0, 25, 1000])
+def test_gradient_after_other_calls(pdl, segment):
+    """Calls with other models, lengths and receivers between a forward run and its gradient:
+    the gradient is that of its own run, bit for bit."""
+    import torch
+    from das_gb300.autograd import model_traces
+    from das_gb300.rtm_engine import TSWRTMEngine
+    from das_gb300.velocity_flood import FloodModels
+    from das_gb300.wave_solver import WaveSolver2D
+    nt = 120
+    rng = np.random.default_rng(9)
+    v, v2 = (rng.uniform(1500, 3000, (NZ, NX)).astype(np.float32) for _ in range(2))
+    w, w2 = (rng.standard_normal(n).astype(np.float32) for n in (nt, 40))
+    rix = np.arange(4, NX - 4, 9)
+    r = torch.tensor(rng.standard_normal((nt, len(rix))).astype(np.float32), device="cuda")
+    d2 = rng.standard_normal((40, NX)).astype(np.float32)
+    s = WaveSolver2D(NX, NZ, 5.0, 5.0, 5e-4, n_sponge=12)
+    s.set_launch("grid", pdl)
+    s.set_checkpoint_segment(segment)
+    grads = []
+    for between in (0, 1, 2, 3):
+        vt = torch.tensor(v, device="cuda", requires_grad=True)
+        d = model_traces(vt, s, w, NX // 3, 2, rix, 3)
+        if between & 1:
+            s.forward_propagate_acoustic(v2, w2, 50, 1, np.arange(NX), 2)
+        if between & 2:
+            TSWRTMEngine(s, "checkpoint").migrate_shot(FloodModels(v2, v2, v2, 0, 0), w2, 70, 4,
+                                                       d2, np.arange(NX), 5, 2)
+        d.backward(r)
+        grads.append(vt.grad.cpu().numpy())
+    s.close()
+    assert np.abs(grads[0]).max() > 0
+    for g in grads[1:]:
+        np.testing.assert_array_equal(grads[0], g)

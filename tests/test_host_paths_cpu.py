@@ -1,5 +1,7 @@
 """What the engines' host code launches, captures and allocates, on a stand-in CUDA runtime
 (no GPU, no arithmetic)."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -220,3 +222,29 @@ def test_kept_states_make_room_for_snapshots(fake):
 
 def _lib_check(lib, rc):
     assert rc == 0, lib.w2d_last_error()
+
+
+class _ShotHead(ctypes.Structure):
+    """The first fields of the resident kernel's RsShot."""
+    _fields_ = [(n, ctypes.c_int) for n in ("nx", "nz", "ldx", "gx", "gz", "maxc", "maxr")] + \
+               [("inv_dx2", ctypes.c_float), ("inv_dz2", ctypes.c_float), ("fs", ctypes.c_int),
+                ("n_sponge", ctypes.c_int), ("lut", ctypes.c_void_p)] + \
+               [(n, ctypes.c_int) for n in ("src_ix", "src_iz", "rec_iz", "n_rec", "rec_c0")]
+
+
+@pytest.mark.parametrize("segment", [0, 25, 1000])
+def test_gradient_after_other_calls_uses_its_own_receivers(fake, segment):
+    """The residuals of a gradient are (nt, n_rec) of its own forward run: with the receivers
+    of a call in between, the adjoint would index them past their end."""
+    from das_gb300.wave_solver import WaveSolver2D
+    nz, nx, nt = 150, 700, 300
+    s = WaveSolver2D(nx, nz, 5.0, 5.0, 5e-4)
+    s.set_checkpoint_segment(segment)
+    assert _fwi_forward(fake, s, nt) == 0
+    s.forward_propagate_acoustic(_vel(nz, nx), np.zeros(10, np.float32), 100, 7, np.arange(nx), 9)
+    head, p = _ShotHead(), np.zeros(1, np.float32)
+    for _ in range(2):
+        _lib_check(fake, fake.w2d_fwi_gradient(s._eng(), p.ctypes.data, p.ctypes.data))
+        fake.fake_last_cooperative(ctypes.byref(head), ctypes.sizeof(head))
+        assert (head.nx, head.nz, head.n_rec, head.rec_iz, head.rec_c0) == (nx, nz, 4, 2, 2)
+    s.close()
