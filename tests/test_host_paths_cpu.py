@@ -248,3 +248,56 @@ def test_gradient_after_other_calls_uses_its_own_receivers(fake, segment):
         fake.fake_last_cooperative(ctypes.byref(head), ctypes.sizeof(head))
         assert (head.nx, head.nz, head.n_rec, head.rec_iz, head.rec_c0) == (nx, nz, 4, 2, 2)
     s.close()
+
+
+def test_tune_plain_times_the_step_kernels(fake, tmp_path, monkeypatch):
+    """A grid that fits the chip ignores the tile unless the call runs one launch per step:
+    the tiles are timed on such a call."""
+    from das_gb300 import autotune
+    from das_gb300.wave_solver import WaveSolver2D
+    monkeypatch.setenv("DAS_GB300_TUNE_CACHE", str(tmp_path / "tune.json"))
+    s = WaveSolver2D(400, 150, 5.0, 5.0, 5e-4)
+    autotune.tune_plain(s, _vel(150, 400), nt_sample=50)
+    n = fake_device.counts(fake)
+    assert n["cooperative"] == 0 and n["graph"] == 2 * len(autotune.PLAIN_TILES)
+    s.close()
+
+
+def test_tune_batch_compares_tiles_on_step_kernels(tmp_path, monkeypatch):
+    """Where the shots run on chip in the grid form (no two receivers in a column) the times of
+    its tiles differ by noise alone: the tile is the one that is fastest in step kernels."""
+    import das_gb300.batch as batch
+    from das_gb300 import autotune
+    from das_gb300.batch import ShotJob
+    monkeypatch.setenv("DAS_GB300_TUNE_CACHE", str(tmp_path / "tune.json"))
+    noise = iter([1.0, 1.02, 1.01] + [1.0] * 100)
+
+    class StandIn:
+        def __init__(self, arena_bytes, max_shots, tile, steps_per_launch, launches_per_graph,
+                     form):
+            self.form, self.tile = form, tuple(tile)
+
+        def run(self, jobs):
+            shared = any(len(set(np.asarray(j.receiver_ix).tolist())) < len(j.receiver_ix)
+                         for j in jobs)
+            for j in jobs:
+                assert j.data.shape == (len(j.wavelet), len(j.receiver_ix))
+            if self.form == "queue":
+                ms = 9.0
+            elif shared:
+                ms = {(4, 4): 3.0, (8, 4): 2.5, (4, 8): 4.0}[self.tile]
+            else:
+                ms = next(noise) if len(jobs) > 2 else 1.0
+            return [], {"counted_points": 1e6 * len(jobs), "device_ms": ms}
+
+        def close(self):
+            pass
+
+    monkeypatch.setattr(batch, "BatchEngine", StandIn)
+    v = _vel(40, 60)
+    for n_rec in (60, 0):
+        jobs = [ShotJob(60, 40, 5.0, 5.0, 5e-4, v, v, np.zeros(99, np.float32),
+                        np.zeros((99, n_rec), np.float32), np.arange(n_rec), 30, 2, 2, 2, 10,
+                        0.0015, True) for _ in range(5)]
+        cfg, table = autotune.tune_batch(jobs, use_cache=False)
+        assert cfg == ((8, 4), 16, 16, "grid") and len(table) == len(autotune.BATCH_CANDIDATES)
