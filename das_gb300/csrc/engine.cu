@@ -439,11 +439,11 @@ AcStep base_step(w2d_engine* e)
     return s;
 }
 
-// Whether the steps of a pass run in the resident form: the default launch mode, a grid
-// that fits the chip, and a source and receivers that the kernel takes.
-bool resident(const w2d_engine* e, int n_rec, bool with_source)
+// Whether the steps of a pass of nt run in the resident form: the default launch mode, a grid
+// that fits the chip, a source and receivers that the kernel takes, and steps worth it.
+bool resident(const w2d_engine* e, int nt, int n_rec, bool with_source)
 {
-    return e->rs.ok() && !e->persistent && e->pdl && !e->two_step && !e->l2_hints &&
+    return nt >= RS_MIN_STEPS && e->rs.ok() && !e->persistent && e->pdl && !e->two_step && !e->l2_hints &&
            rs_shot_fits(e->nx, e->nz, with_source ? e->h_shot[0] : -1, e->h_shot[1], n_rec,
                         e->h_shot[2], e->one_per_column);
 }
@@ -1054,7 +1054,7 @@ int w2d_forward(w2d_engine* e, int vel_slot, const float* wavelet, int nt, int s
     e->last_storage = 0;
     const float dt2inj = (float)(e->dt_d * e->dt_d);
     cudaEventRecord(e->ev0, e->stream);
-    const bool on_chip = resident(e, n_rec, true);
+    const bool on_chip = resident(e, nt, n_rec, true);
     auto pass = [&]() -> int {
         int r;
         if ((r = forward_begin(e, dt2inj))) return r;
@@ -1125,7 +1125,7 @@ int w2d_backward_correlate(w2d_engine* e, int vel_slot, const float* data, int n
     const float dt2inj = (float)(e->dt_d * e->dt_d);
     const float img_dt = (float)(e->dt_d * (double)snapshot_interval);
     cudaEventRecord(e->ev0, e->stream);
-    const bool on_chip = resident(e, n_rec, false);
+    const bool on_chip = resident(e, nt, n_rec, false);
     auto pass = [&]() -> int {
         int r;
         if (n_rec > 0) {
@@ -1200,7 +1200,7 @@ int migrate_core(w2d_engine* e, int nt, int n_rec, int snapshot_interval, int st
 
     // The form of each pass's steps, decided here for the whole migration: the backward
     // pass has no source and may run on chip where the forward one does not.
-    const bool fwd_chip = resident(e, n_rec, true), bwd_chip = resident(e, n_rec, false);
+    const bool fwd_chip = resident(e, nt, n_rec, true), bwd_chip = resident(e, nt, n_rec, false);
 
     // 1. forward pass in slot 0 with illumination
     auto forward = [&]() -> int {
@@ -1677,9 +1677,9 @@ bool written_cell(const w2d_engine* e, int iz, int ix)
 
 // Whether the gradient runs in the resident form: when the passes do (receivers on interior
 // rows then sit on interior cells), and the per-cell adjoint was not asked for.
-bool fwi_resident(const w2d_engine* e, int n_rec)
+bool fwi_resident(const w2d_engine* e, int nt, int n_rec)
 {
-    return !e->adj_cells && resident(e, n_rec, true);
+    return !e->adj_cells && resident(e, nt, n_rec, true);
 }
 
 }  // namespace
@@ -1734,7 +1734,7 @@ int fwi_plan(w2d_engine* e, w2d_fwi_state* f, bool keep_all)
     const size_t all = (size_t)nt * e->plane;
     const size_t room = e->budget ? (size_t)e->budget / 8
                                   : std::max(free_budget(e) / 8, f->segbuf.cap * 4);
-    const bool keep = keep_all && e->fwi_seg <= 0 && fwi_resident(e, f->n_rec) &&
+    const bool keep = keep_all && e->fwi_seg <= 0 && fwi_resident(e, f->nt, f->n_rec) &&
                       all * 4 <= room && f->segbuf.ensure(all) == W2D_OK;
     // what a run before this one kept and this one does not goes back
     if (!keep && fwi_kept(f)) f->segbuf.release();
@@ -1742,7 +1742,7 @@ int fwi_plan(w2d_engine* e, w2d_fwi_state* f, bool keep_all)
     if (keep) f->seg = nt;
     f->n_seg = (nt + f->seg - 1) / f->seg;
     f->stored = f->seg >= nt;
-    f->lap = f->stored && fwi_resident(e, f->n_rec);
+    f->lap = f->stored && fwi_resident(e, f->nt, f->n_rec);
     if ((rc = f->segbuf.ensure((size_t)f->seg * e->plane)) ||
         (rc = e->ckpt.ensure((size_t)f->n_seg * 3 * e->plane)))
         return rc;
@@ -1769,7 +1769,7 @@ int fwi_run_forward(w2d_engine* e, w2d_fwi_state* f, float* rec_out)
         o.ckpt = e->ckpt.p;
         o.ckpt_every = f->seg;
     }
-    return run_forward_steps(e, 0, o, 0, f->nt, resident(e, f->n_rec, true), dt2inj);
+    return run_forward_steps(e, 0, o, 0, f->nt, resident(e, f->nt, f->n_rec, true), dt2inj);
 }
 
 }  // namespace
@@ -1875,7 +1875,7 @@ int w2d_fwi_gradient(w2d_engine* e, const float* resid_dev, float* grad_dev)
                                  cudaMemcpyDeviceToDevice, e->stream));
     if ((rc = zero_pass(e, 1))) return rc;
     W2D_CUDA_TRY(cudaMemsetAsync(f->grad_c.p, 0, plane_b, e->stream));
-    if (f->stored ? f->lap : fwi_resident(e, n_rec)) {
+    if (f->stored ? f->lap : fwi_resident(e, nt, n_rec)) {
         // q[nt] from the last residuals; then, segment by segment, L P recomputed and the
         // adjoint imaged with it
         e->last_launches = 0;
@@ -1972,7 +1972,7 @@ int w2d_fwi_gradient(w2d_engine* e, const float* resid_dev, float* grad_dev)
             r.interval = 1;
             r.snaps = f->segbuf.p;
             r.slot0 = a;
-            if ((rc = run_forward_steps(e, 0, r, a, b, resident(e, n_rec, true), dt2inj))) return rc;
+            if ((rc = run_forward_steps(e, 0, r, a, b, resident(e, nt, n_rec, true), dt2inj))) return rc;
             e->last_recompute += b - a;
             adj_chain = false;  // the segment's first adjoint step waits for the stream
         }

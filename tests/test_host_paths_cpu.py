@@ -301,3 +301,26 @@ def test_tune_batch_compares_tiles_on_step_kernels(tmp_path, monkeypatch):
                         0.0015, True) for _ in range(5)]
         cfg, table = autotune.tune_batch(jobs, use_cache=False)
         assert cfg == ((8, 4), 16, 16, "grid") and len(table) == len(autotune.BATCH_CANDIDATES)
+
+
+@pytest.mark.parametrize("nt", [1, 2, 5, 6, 40])
+def test_short_passes_keep_the_step_kernels(fake, nt):
+    """Loading a grid onto the chip costs more than a few launches."""
+    from das_gb300.rtm_engine import TSWRTMEngine
+    from das_gb300.velocity_flood import FloodModels
+    from das_gb300.wave_solver import WaveSolver2D
+    nz, nx = 150, 400
+    s = WaveSolver2D(nx, nz, 5.0, 5.0, 5e-4)
+    v, w, d = _vel(nz, nx), np.zeros(nt, np.float32), np.zeros((nt, nx), np.float32)
+    s.forward_propagate_acoustic(v, w, nx // 2, 2, np.arange(nx), 2)
+    n = fake_device.counts(fake)
+    assert (n["cooperative"], n["captures"]) == ((1, 0) if nt >= 6 else (0, 1))
+    TSWRTMEngine(s, "all").migrate_shot(FloodModels(v, v, v, 0, 0), w, nx // 2, 2, d,
+                                        np.arange(nx), 2, 2)
+    n = fake_device.counts(fake)
+    assert (n["cooperative"], n["captures"]) == ((2, 0) if nt >= 6 else (0, 2))
+    _lib_check(fake, _fwi_forward(fake, s, nt))
+    p = np.zeros(1, np.float32)
+    _lib_check(fake, fake.w2d_fwi_gradient(s._eng(), p.ctypes.data, p.ctypes.data))
+    assert (fake_device.counts(fake)["cooperative"] > 0) == (nt >= 6)
+    s.close()
