@@ -15,9 +15,10 @@ per shot (forward + backward; recomputation not counted).
   in page-locked memory; the host->device copies of the gather, wavelet and both
   velocity models and the device->host copies of image and illumination are
   inside the timed region.
-* ``roofline``: the algorithmic bytes of all time steps in the timed region over the
-  device time of the region, against the measured HBM copy bandwidth; per launch where
-  each step is one, per step where one launch runs a whole pass on chip.
+* ``roofline``: where a whole pass is one launch (wavefields on chip), the float32 operations
+  of all time steps in the timed region over the device time of the region, against the
+  measured rate of such operations; where each step is a launch, their algorithmic bytes
+  against the measured HBM copy bandwidth.
 * ``cpu_baseline``: the reference's CPU path (wave2d.c + its Python time loops,
   restated in oracle/) timed on this host's cores over a bounded sample.
 * ``--impl reference``: that CPU implementation alone, each step a bounded sample
@@ -117,6 +118,19 @@ def measured_peaks():
             d = json.load(f)
         return float(d["hbm_gbs"]), "measured"
     return 6800.0, "fallback"
+
+
+# float32 operations a second: independent rounded adds, or multiplies, measured on a GB300 at
+# 2070 MHz (36.6e12 where the two take turns; no fused ones, which the bit-exact time loop and
+# its oracle do not use)
+FP32_OPS = 39.1e12
+
+
+def ops_per_shot(sv, interval):
+    """float32 operations of one migration: 20 a point and step of either pass; 2 more a point
+    where a forward step adds to the illumination, 3 where a backward step images."""
+    n_snaps = (sv.nt - 1) // interval + 1
+    return sv.nz * sv.nx * (2 * sv.nt * 20 + n_snaps * 5)
 
 
 def committed_traffic(key="traffic_bytes_per_launch", profile="acoustic_step_large_plain.md"):
@@ -411,11 +425,35 @@ def run_ours(args, dist):
     peak, peak_kind = measured_peaks()
     step_launches_per_shot = 2 * sv.nt + recompute // max(K, 1)
     on_chip = launches < 2 * sv.nt  # one launch advanced many steps
-    algo_bytes = bytes_per_shot(sv, interval) * K + recompute * sv.nz * sv.nx * 16
-    achieved = algo_bytes / (ms.value / 1e3) / 1e9
-    per_launch = algo_bytes / (step_launches_per_shot * K)
-    traffic = (committed_traffic("traffic_bytes_per_step", "resident_loop_large.md") if on_chip
-               else committed_traffic())
+    if on_chip:
+        algo_ops = ops_per_shot(sv, interval) * K + recompute * sv.nz * sv.nx * 20
+        achieved = algo_ops / (ms.value / 1e3) / 1e12
+        roofline = {
+            "bound": "fp32", "achieved": achieved, "peak": FP32_OPS / 1e12, "unit": "Tops/s",
+            "frac": achieved / (FP32_OPS / 1e12),
+            "peak_source": "measured rate of independent float32 operations",
+            "traffic": committed_traffic("traffic_bytes_per_step", "resident_loop_large.md"),
+            "limiter": "issue slots: the wavefields and the model stay in shared and tensor "
+                       "memory for a whole pass, about half the slots are used (fixed latency, "
+                       "shared memory, math pipe stalls about alike), and DRAM carries the "
+                       "snapshots alone (traffic: DRAM bytes per step, from a pass without "
+                       "snapshots, which add 16 MB each)",
+            "kernel": "acoustic_resident_kernel (a whole pass per launch)",
+            "operations_per_step": algo_ops / (step_launches_per_shot * K)}
+    else:
+        algo_bytes = bytes_per_shot(sv, interval) * K + recompute * sv.nz * sv.nx * 16
+        achieved = algo_bytes / (ms.value / 1e3) / 1e9
+        roofline = {
+            "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
+            "frac": achieved / peak, "peak_source": f"{peak_kind} hbm_gbs",
+            "traffic": committed_traffic(),
+            "traffic_cold": committed_traffic("cold_traffic_bytes_per_launch"),
+            "limiter": "latency: the three wave planes and the model (64 MB) stay in L2 from "
+                       "step to step, so DRAM carries the snapshot stream and write-backs "
+                       "(traffic: warm-cache ncu, per launch) and each CTA waits on its own "
+                       "TMA round trip; frac is algorithmic bytes over the HBM copy rate",
+            "kernel": "acoustic_step_kernel (fused forward / backward+imaging)",
+            "algorithmic_bytes_per_launch": algo_bytes / (step_launches_per_shot * K)}
 
     # end-to-end through the public drop-in call, inputs in page-locked host memory
     ke = max(1, min(K, args.e2e_steps))
@@ -471,28 +509,7 @@ def run_ours(args, dist):
                "shots_per_s": K * dist.world / dev_s,
                "recomputed_steps_per_shot": recompute / max(K, 1),
                "device_memory_in_use_gb": (total_b - free_b) / 1e9,
-               "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                            "frac": achieved / peak, "traffic": traffic,
-                            "traffic_cold": (None if on_chip else
-                                             committed_traffic("cold_traffic_bytes_per_launch")),
-                            "limiter": "issue slots: the wavefields and the model stay in "
-                                       "shared and tensor memory for a whole pass, so DRAM "
-                                       "carries the snapshots alone (traffic: per step, from a "
-                                       "pass without snapshots, which add 16 MB each); frac is "
-                                       "the bytes a launch per step would move over the HBM "
-                                       "copy rate" if on_chip else
-                                       "latency: the three wave planes and the model (64 MB) "
-                                       "stay in L2 from step to step, so DRAM carries the "
-                                       "snapshot stream and write-backs (traffic: warm-cache "
-                                       "ncu, per launch) and each CTA waits on its own TMA "
-                                       "round trip; frac is algorithmic bytes over the HBM "
-                                       "copy rate",
-                            "peak_source": f"{peak_kind} hbm_gbs",
-                            "kernel": ("acoustic_resident_kernel (a whole pass per launch)" if on_chip else
-                                       "acoustic_step_kernel (fused forward / backward+imaging)"),
-                            "algorithmic_bytes_per_launch": (
-                                algo_bytes / max(launches, 1) if on_chip else per_launch),
-                            "algorithmic_bytes_per_step": per_launch},
+               "roofline": roofline,
                "e2e": {"value": e2e, "unit": UNIT, "h2d_bytes_per_step": int(h2d),
                        "d2h_bytes_per_step": int(d2h), "steps": ke,
                        "per_call_ms": [round(c, 2) for c, _ in calls],
@@ -610,14 +627,25 @@ def run_batched(args, dist):
                       f"nt={min(args.cpu_nt, len(jobs[0].wavelet))}: {rate:.2f} Gpts/s in "
                       f"{el:.1f} s, extrapolated to the {len(jobs)} gathers' {pts / 1e12:.2f} T "
                       f"counted points"}
-    # roofline of the batch kernel at the device rate: 22 algorithmic bytes per counted
-    # point at snapshot interval 2 (16 per step; every second forward step adds 12 for the
-    # snapshot and illumination, every second backward step 12 for the imaging)
-    peak, peak_kind = measured_peaks()
-    dev = out["gpts_per_s_device"] * 1e9 * 22.0 / 1e9
-    out["roofline"] = {"bound": "hbm", "achieved": dev, "peak": peak, "unit": "GB/s",
-                       "frac": dev / peak, "peak_source": f"{peak_kind} hbm_gbs",
-                       "kernel": "acoustic_batch_step_kernel", "bytes_per_counted_point": 22.0}
+    if st["launches"] < max(2 * len(j.wavelet) for j in jobs):
+        # many steps a launch (shots on chip): 20 operations a point and step, 2 more where a
+        # forward step adds to the illumination, 3 where a backward step images (interval 2)
+        ops = out["gpts_per_s_device"] * 1e9 * (20.0 + 5.0 / 4.0) / 1e12
+        out["roofline"] = {"bound": "fp32", "achieved": ops, "peak": FP32_OPS / 1e12,
+                           "unit": "Tops/s", "frac": ops / (FP32_OPS / 1e12),
+                           "peak_source": "measured rate of independent float32 operations",
+                           "kernel": "acoustic_resident_kernel (shots in waves)",
+                           "operations_per_counted_point": 21.25}
+    else:
+        # the batch step kernel: 22 algorithmic bytes per counted point at snapshot interval 2
+        # (16 per step; every second forward step adds 12 for the snapshot and illumination,
+        # every second backward step 12 for the imaging)
+        peak, peak_kind = measured_peaks()
+        dev = out["gpts_per_s_device"] * 1e9 * 22.0 / 1e9
+        out["roofline"] = {"bound": "hbm", "achieved": dev, "peak": peak, "unit": "GB/s",
+                           "frac": dev / peak, "peak_source": f"{peak_kind} hbm_gbs",
+                           "kernel": "acoustic_batch_step_kernel",
+                           "bytes_per_counted_point": 22.0}
     _emit(out)
 
 
@@ -705,6 +733,7 @@ def run_elastic(args, dist):
     times = []
     fwd_ms, grad_ms = [], []
     v = torch.tensor(vs_mig, device="cuda", requires_grad=True)
+    free0 = torch.cuda.mem_get_info()[0]
     for k, six in enumerate(order):
         if k == W:
             v.grad = None  # the survey gradient sums the timed shots only
@@ -719,6 +748,8 @@ def run_elastic(args, dist):
             times.append(time.perf_counter() - t0)
             fwd_ms.append(f_ms)
             grad_ms.append(solver.last_ms)
+    # every forward state kept, or checkpoints and recomputation: by what the solver holds
+    kept = free0 - torch.cuda.mem_get_info()[0] >= 0.5 * 20.0 * nz * nx * nt
     g = v.grad.detach()
     survey = {"shots": K, "distinct_sources": len(set(order[W:])),
               "gradient_finite": bool(torch.isfinite(g).all().item()),
@@ -727,16 +758,19 @@ def run_elastic(args, dist):
     # roofline of the gradient phase (the device time of J.backward): per time step and
     # grid point the recomputation moves 56 B (the forward step: five fields read and
     # written, lambda, mu and the two buoyancies read) + 20 B (the five fields stored
-    # into the segment), and the two tiled adjoint passes 27 + 9 planes = 144 B
+    # into the segment), unless the forward run kept its states; and the two tiled adjoint
+    # passes 27 + 9 planes = 144 B
     peak, peak_kind = measured_peaks()
-    grad_bytes = nz * nx * nt * (56 + 20 + 144)
+    per_pt = 144 if kept else 56 + 20 + 144
+    grad_bytes = nz * nx * nt * per_pt
     achieved = grad_bytes / (statistics.mean(grad_ms) / 1e3) / 1e9
     fwd_achieved = nz * nx * nt * 56 / (statistics.mean(fwd_ms) / 1e3) / 1e9
     out = {"metric": "elastic RTM gradient Gpts/s", "value": pts * K / sum(times) / 1e9,
            "unit": "Gpts/s", "n_gpus": 1, "higher_is_better": True, "dtype": "f32",
            "data": "synthetic", "steps": K, "warmup": W,
            "config": {"workload": f"elastic velocity-stress gradient 1024x2048, dx 2 m, nt {nt}, "
-                                  f"{len(rix)} vertical-strain receivers, 5 Hz, checkpointed, "
+                                  f"{len(rix)} vertical-strain receivers, 5 Hz, "
+                                  f"{'states kept' if kept else 'checkpointed'}, "
                                   f"{K} shots over the 64 surface sources into one gradient",
                       "adjoint": args.el_adjoint, "tiles": args.el_tiles},
            "s_per_shot": sum(times) / K, "survey": survey,
@@ -746,9 +780,10 @@ def run_elastic(args, dist):
            "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                         "frac": achieved / peak, "traffic": None,
                         "peak_source": f"{peak_kind} hbm_gbs",
-                        "kernel": "gradient phase: el_adj_a + el_adj_b (tiled adjoint passes) "
-                                  "and the segment recomputation's step kernels",
-                        "algorithmic_bytes_per_step_point": 56 + 20 + 144,
+                        "kernel": "gradient phase: el_adj_a + el_adj_b (tiled adjoint passes)" +
+                                  ("" if kept else
+                                   " and the segment recomputation's step kernels"),
+                        "algorithmic_bytes_per_step_point": per_pt,
                         "forward_phase_achieved_gbs": fwd_achieved,
                         "forward_phase_frac": fwd_achieved / peak}}
     _emit(out)
@@ -757,9 +792,9 @@ def run_elastic(args, dist):
 def run_gradient(args, dist):
     """Acoustic velocity gradient (the differentiable form): the 1000 x 4000 grid, nt 8000,
     receivers on every written column of row 2; per step one shot's forward modelling
-    through ``das_gb300.autograd`` and the misfit's backward (the hand-written adjoint
-    kernel over the forward wavefield recomputed segment by segment from checkpoints),
-    accumulated into one gradient over the shots of the run."""
+    through ``das_gb300.autograd`` and the misfit's backward (the adjoint over the forward
+    states, kept or recomputed segment by segment from checkpoints), accumulated into one
+    gradient over the shots of the run."""
     import torch
     from das_gb300.autograd import model_traces
     from das_gb300.wave_solver import WaveSolver2D
@@ -793,35 +828,52 @@ def run_gradient(args, dist):
             fwd_s.append(t1 - t0)
             grad_s.append(t2 - t1)
             times.append(t2 - t0)
-    recomputed = s.last_stats()["recomputed_steps"]
+    st = s.last_stats()
+    recomputed, on_chip = st["recomputed_steps"], st["step_launches"] < nt
     g = v.grad.detach()
     s.close()
     pts = 2.0 * nz * nx * nt
-    # gradient phase per time step and grid point: the recomputed forward step (16 B) and
-    # its store into the segment (4 B), the adjoint step (a[n+1], c, P[n], a[n+2] read,
-    # a[n] written: 20 B) and the gradient's read-modify-write (8 B)
-    peak, peak_kind = measured_peaks()
-    per_pt = 16 + 4 + 20 + 8
-    achieved = nz * nx * nt * per_pt / statistics.mean(grad_s) / 1e9
-    fwd_achieved = nz * nx * nt * 16 / statistics.mean(fwd_s) / 1e9
+    n = nz * nx * nt
+    if on_chip:
+        # operations per point: 20 an adjoint step and 3 for the gradient's sum, 20 a
+        # recomputed step; 20 a forward step
+        ops = n * 23 + nz * nx * recomputed * 20
+        achieved = ops / statistics.mean(grad_s) / 1e12
+        roofline = {"bound": "fp32", "achieved": achieved, "peak": FP32_OPS / 1e12,
+                    "unit": "Tops/s", "frac": achieved / (FP32_OPS / 1e12), "traffic": None,
+                    "peak_source": "measured rate of independent float32 operations",
+                    "kernel": "gradient phase: acoustic_resident_kernel, adjoint and recomputed "
+                              "segments (host-timed phase)",
+                    "forward_phase_achieved_tops": n * 20 / statistics.mean(fwd_s) / 1e12,
+                    "forward_phase_frac": n * 20 / statistics.mean(fwd_s) / FP32_OPS}
+    else:
+        # gradient phase per time step and grid point: the recomputed forward step (16 B) and
+        # its store into the segment (4 B), the adjoint step (a[n+1], c, P[n], a[n+2] read,
+        # a[n] written: 20 B) and the gradient's read-modify-write (8 B)
+        peak, peak_kind = measured_peaks()
+        per_pt = 16 + 4 + 20 + 8
+        achieved = n * per_pt / statistics.mean(grad_s) / 1e9
+        fwd_achieved = n * 16 / statistics.mean(fwd_s) / 1e9
+        roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
+                    "frac": achieved / peak, "traffic": None,
+                    "peak_source": f"{peak_kind} hbm_gbs",
+                    "kernel": "gradient phase: acoustic_adjoint_kernel and the segment "
+                              "recomputation's step kernels (host-timed phase)",
+                    "algorithmic_bytes_per_step_point": per_pt,
+                    "forward_phase_achieved_gbs": fwd_achieved,
+                    "forward_phase_frac": fwd_achieved / peak}
     _emit({"metric": "acoustic RTM gradient Gpts/s", "value": pts * K / sum(times) / 1e9,
            "unit": "Gpts/s", "n_gpus": 1, "higher_is_better": True, "dtype": "f32",
            "data": "synthetic", "steps": K, "warmup": W,
            "config": {"workload": f"acoustic velocity gradient {nz}x{nx}, nt {nt}, {len(rix)} "
-                                  f"receivers, checkpointed; {K} shots into one gradient"},
+                                  f"receivers, {'checkpointed' if recomputed else 'states kept'}; "
+                                  f"{K} shots into one gradient"},
            "s_per_shot": sum(times) / K, "s_forward": statistics.mean(fwd_s),
            "s_gradient": statistics.mean(grad_s), "recomputed_steps_per_shot": recomputed,
            "counted_points_per_shot": pts,
            "gradient": {"finite": bool(torch.isfinite(g).all().item()),
                         "max_abs": float(g.abs().max().item())},
-           "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                        "frac": achieved / peak, "traffic": None,
-                        "peak_source": f"{peak_kind} hbm_gbs",
-                        "kernel": "gradient phase: acoustic_adjoint_kernel and the segment "
-                                  "recomputation's step kernels (host-timed phase)",
-                        "algorithmic_bytes_per_step_point": per_pt,
-                        "forward_phase_achieved_gbs": fwd_achieved,
-                        "forward_phase_frac": fwd_achieved / peak}})
+           "roofline": roofline})
 
 
 def run_served(args, dist):
@@ -835,8 +887,8 @@ def run_served(args, dist):
                           args.serve_nt_scale)
     n_el = sum(r.kind == "elastic" for r in trace)
     tile = tuple(int(t) for t in (args.tile or "4,4").split(","))
-    # the elastic workers hold up to ~17 GB each (checkpoints and one recomputed segment
-    # of a 1024 x 4096, nt 8000 grid): leave them room beside the acoustic arena
+    # the elastic workers hold up to their budget of 20 GB each (the states of a batch, or
+    # checkpoints and one recomputed segment): leave them room beside the acoustic arena
     eng = BatchEngine(arena_bytes=int(min(args.arena_gb, 160.0) * (1 << 30)), max_shots=4096,
                       tile=tile, steps_per_launch=args.spl, launches_per_graph=args.lpg,
                       form=args.batch_form)

@@ -954,9 +954,9 @@ int w2d_batch_launch(w2d_batch* b)
     if (b->form == 1) {
         // The waves of the shots that fit the chip; then S * chunks launches, one phase step
         // of every other active shot each, and one advance of all shots' progress, replayed
-        // as one captured graph.  (20 gathers of 200-600 x 400-2000,
-        // 1500-3000 steps, host arrays in and out: 329 ms a batch with step kernels alone, 155
-        // with waves and the result arrays made ready meanwhile; 20 shots of 150 x 400, 2000 steps: 52 and 22.)
+        // as one captured graph.  (20 gathers of 200-600 x 400-2000, 1500-3000 steps, host
+        // arrays in and out: 329 ms a batch with step kernels alone, 155 with waves and the
+        // result arrays made ready meanwhile; 20 shots of 150 x 400, 2000 steps: 52 and 22.)
         const int steps = b->S * b->chunks;
         const long long key =
             (((long long)b->t_all * 65536 + (long long)b->n_step) * 4096 + steps) * 256 +

@@ -43,7 +43,8 @@
 // are resident at once (cooperative launch).
 //
 // Arithmetic: the reference's operation order with every operation rounded (no
-// contraction), as in acoustic_kernels.cuh, so the results are bit-identical to it.
+// contraction), as in acoustic_kernels.cuh, so finite results are bit-identical to it but for
+// the sign of a zero (2c - p_prev is formed as -(p_prev - 2c), see rs_stencil).
 // Cells the reference never writes stay zero unless receivers inject into them: the
 // source and the receivers' row must lie on interior rows (rs_shot_fits), so the only
 // such cells are the four of that row beside the left and right edges.  Their values in
@@ -218,7 +219,8 @@ __device__ __forceinline__ F4 rs_stencil(const RsConst& k, const F4& w0, const F
                               kca), k.dz2);
     const f32x2 zb = mul(add2(add2(mul(k.k2, add2(w0.b, w4.b)), mul(k.k1, add2(w1.b, w3.b))),
                               kcb), k.dz2);
-    // v*lap + (2c - pp), the second term as -(pp - 2c): 2c is exact, so one rounding
+    // v*lap + (2c - pp), the second term as -(pp - 2c): 2c is exact, so one rounding.  (Where
+    // 2c overflows the Laplacian has: the cell is infinite or NaN in either form.)
     lap.a = add2(xa, za);
     lap.b = add2(xb, zb);
     F4 u;
@@ -378,8 +380,8 @@ __device__ __forceinline__ F4 rs_frame(const F4& u, const float4& fx, float fz, 
 // leaves next to no L1): the rest is read from the tile's record.
 struct RsMine {
     // edge unit: row, unit column << 16, and whether there is one (bit 31), it is written
-    // (bit 30), a rule of its own applies (bit 29), it is the last column's (bit 28); packets it sends along x and z,
-    // as indices into the packet buffer, -1: none
+    // (bit 30), a rule of its own applies (bit 29), it is the last column's (bit 28); packets it
+    // sends along x and z, as indices into the packet buffer, -1: none
     unsigned e;
     int ox, oz;
     // interior units: unit column, first row << 8, number of rows << 24 (0: none)
