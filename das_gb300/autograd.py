@@ -5,9 +5,9 @@ receiver_iz)`` returns the receiver traces (nt, n_rec) that
 ``WaveSolver2D.forward_propagate_acoustic`` would record in ``vel`` (the same
 forward kernels), as a CUDA tensor.  Its backward runs the hand-written adjoint
 (the resident loop where the grid fits the chip, else ``acoustic_adjoint_kernel``)
-over the forward states, kept where they fit or recomputed segment by segment from
-checkpoints, and returns dL/dvel: for a least-squares misfit this is the velocity gradient, i.e. the adjoint-state
-migration image of the data residual.
+over the forward states, kept where they fit or recomputed segment by segment
+from checkpoints, and returns dL/dvel: for a least-squares misfit this is the
+velocity gradient, i.e. the adjoint-state migration image of the data residual.
 
 PyTorch is used only for this wrapper (tensors, autograd); the arithmetic runs
 in ``libwave2d_cuda.so`` on the tensors' device memory.

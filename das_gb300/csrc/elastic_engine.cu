@@ -322,8 +322,9 @@ int w2d_elastic_forward_batch(w2d_elastic* e, int n_shots, const float* lam, con
     plan_segments(nt, &e->seg_len, &e->n_seg);
     const size_t P = e->plane, SS = e->SS();
     // Every state kept where they all fit an eighth of the free memory (the rest stays for
-    // others), or the whole batch with them the budget: nothing is recomputed (forward and gradient, 4 shots of 363 x 725, 700 steps:
-    // 41.6 -> 31.0 ms; 1024 x 2048, 500 steps: 52.5 -> 41.4).  Not where no gradient follows:
+    // others), or the whole batch with them the budget: nothing is recomputed (forward and
+    // gradient, 4 shots of 363 x 725, 700 steps: 41.6 -> 31.0 ms; 1024 x 2048, 500 steps: 52.5 ->
+    // 41.4).  Not where no gradient follows:
     // a forward pass alone is faster in place, its state in L2 from step to step (the same
     // two: 11.8 ms with the states kept and 11.4 without, 13.0 and 11.2).
     const size_t all = (size_t)(nt + 1) * S * SS;

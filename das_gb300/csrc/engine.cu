@@ -443,7 +443,8 @@ AcStep base_step(w2d_engine* e)
 // that fits the chip, a source and receivers that the kernel takes, and steps worth it.
 bool resident(const w2d_engine* e, int nt, int n_rec, bool with_source)
 {
-    return nt >= RS_MIN_STEPS && e->rs.ok() && !e->persistent && e->pdl && !e->two_step && !e->l2_hints &&
+    return nt >= RS_MIN_STEPS && e->rs.ok() && !e->persistent && e->pdl && !e->two_step &&
+           !e->l2_hints &&
            rs_shot_fits(e->nx, e->nz, with_source ? e->h_shot[0] : -1, e->h_shot[1], n_rec,
                         e->h_shot[2], e->one_per_column);
 }
@@ -1972,7 +1973,8 @@ int w2d_fwi_gradient(w2d_engine* e, const float* resid_dev, float* grad_dev)
             r.interval = 1;
             r.snaps = f->segbuf.p;
             r.slot0 = a;
-            if ((rc = run_forward_steps(e, 0, r, a, b, resident(e, nt, n_rec, true), dt2inj))) return rc;
+            if ((rc = run_forward_steps(e, 0, r, a, b, resident(e, nt, n_rec, true), dt2inj)))
+                return rc;
             e->last_recompute += b - a;
             adj_chain = false;  // the segment's first adjoint step waits for the stream
         }

@@ -14,10 +14,10 @@ constexpr int RS_T = RS_CT + 32;    // and one halo warp: 16 warps, 128 register
 constexpr int RS_MAXR = 15;         // rows of one phase-I thread: its tensor-memory words
 constexpr int RS_SMEM = 227 * 1024; // always the whole SM: no second CTA, which could wait
                                     // for tensor memory while its neighbours wait for it
-// Shortest pass of an engine that runs here: before, loading and storing the tiles takes longer
-// than the launches saved.  us on the device, a launch per step -> here: forward, 40 x 80, 1 step
-// 15.7 -> 24, 4 steps 32 -> 29; 1000 x 4000, 1 step 30 -> 54, 6 steps 80 -> 80; migration, 150 x 400,
-// 2 steps 47 -> 77, 6 steps 90 -> 88; 1000 x 4000, 6 steps 207 -> 213, 8 steps 257 -> 239.
+// Shortest pass of an engine that runs here: loading and storing the tiles of a shorter one takes
+// longer than the launches saved.  us on the device, a launch per step -> here: forward, 40 x 80,
+// 1 step 15.7 -> 24, 4 steps 32 -> 29; 1000 x 4000, 1 step 30 -> 54, 6 steps 80 -> 80; migration,
+// 150 x 400, 2 steps 47 -> 77, 6 steps 90 -> 88; 1000 x 4000, 6 steps 207 -> 213, 8 steps 257 -> 239.
 constexpr int RS_MIN_STEPS = 6;
 constexpr int RS_POLLS = 1 << 21;    // looks at a missing packet before giving up (about 1 s)
 // Groups of 32 packets a warp has in flight: the halo warp, and a compute warp that is done.

@@ -201,18 +201,21 @@ void w2d_host_free(void* p);
 
 /* ---- Differentiable modelling (no reference counterpart: RTM as the adjoint) ----
  * Forward modelling in velocity vel_dev (DEVICE, contiguous nz x nx float32),
- * traces written to traces_dev (DEVICE, nt x n_rec), checkpoints of the forward
- * state kept in the engine.  Source and receivers must sit on written cells
+ * traces written to traces_dev (DEVICE, nt x n_rec), every forward state or
+ * checkpoints kept in the engine.  Source and receivers must sit on written cells
  * (interior, or rows 0/1 with the free surface). */
 int w2d_fwi_forward(w2d_engine* e, const float* vel_dev, const float* wavelet, int nt, int src_ix,
                     int src_iz, const int* rec_ix, int n_rec, int rec_iz, float* traces_dev);
 /* Gradient of sum(resid * traces) with respect to the velocity of the last
  * w2d_fwi_forward on this engine: resid_dev (DEVICE, nt x n_rec), grad_dev
- * (DEVICE, nz x nx, overwritten).  Hand-written adjoint kernel; the forward
- * wavefield is recomputed segment by segment from the checkpoints. */
+ * (DEVICE, nz x nx, overwritten).  Hand-written adjoint over the kept forward states
+ * or over states recomputed segment by segment from the checkpoints; other calls on
+ * the engine may come between the two. */
 int w2d_fwi_gradient(w2d_engine* e, const float* resid_dev, float* grad_dev);
-/* Steps per checkpoint segment of the next w2d_fwi_forward: 0 (the default) picks
- * sqrt(3 nt), the segment length that balances checkpoint and segment storage;
+/* Steps per checkpoint segment of the next w2d_fwi_forward: 0 (the default) keeps
+ * every forward state where the grid runs on chip and they fit an eighth of the memory
+ * at hand (w2d_engine_set_memory_budget), and else picks sqrt(3 nt), the segment
+ * length that balances checkpoint and segment storage;
  * nt or more keeps every forward state of the run (no recomputation, nt planes
  * of device memory).  The gradient is the same bit for bit either way. */
 int w2d_fwi_set_segment(w2d_engine* e, int steps);

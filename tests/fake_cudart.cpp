@@ -4,6 +4,7 @@
 // when it is allocated).
 #include <sys/mman.h>
 
+#include <cstdlib>
 #include <cstring>
 #include <map>
 #include <mutex>
@@ -71,14 +72,27 @@ cudaError_t cudaMemGetInfo(size_t* f, size_t* t)
     *t = total;
     return cudaSuccess;
 }
-cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { return (*p = calloc(n, 1)) ? cudaSuccess : cudaErrorMemoryAllocation; }
+cudaError_t cudaHostAlloc(void** p, size_t n, unsigned)
+{
+    return (*p = calloc(n, 1)) ? cudaSuccess : cudaErrorMemoryAllocation;
+}
 cudaError_t cudaMallocHost(void** p, size_t n) { return cudaHostAlloc(p, n, 0); }
 cudaError_t cudaFreeHost(void* p) { free(p); return cudaSuccess; }
 
 cudaError_t cudaMemcpy(void*, const void*, size_t, cudaMemcpyKind) { return cudaSuccess; }
-cudaError_t cudaMemcpyAsync(void*, const void*, size_t, cudaMemcpyKind, cudaStream_t) { return cudaSuccess; }
-cudaError_t cudaMemcpy2D(void*, size_t, const void*, size_t, size_t, size_t, cudaMemcpyKind) { return cudaSuccess; }
-cudaError_t cudaMemcpy2DAsync(void*, size_t, const void*, size_t, size_t, size_t, cudaMemcpyKind, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaMemcpyAsync(void*, const void*, size_t, cudaMemcpyKind, cudaStream_t)
+{
+    return cudaSuccess;
+}
+cudaError_t cudaMemcpy2D(void*, size_t, const void*, size_t, size_t, size_t, cudaMemcpyKind)
+{
+    return cudaSuccess;
+}
+cudaError_t cudaMemcpy2DAsync(void*, size_t, const void*, size_t, size_t, size_t, cudaMemcpyKind,
+                              cudaStream_t)
+{
+    return cudaSuccess;
+}
 cudaError_t cudaMemset(void*, int, size_t) { return cudaSuccess; }
 cudaError_t cudaMemsetAsync(void*, int, size_t, cudaStream_t) { return cudaSuccess; }
 
@@ -91,7 +105,11 @@ cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { return make(e);
 cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
-cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) { *ms = 1.0f; return cudaSuccess; }
+cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t)
+{
+    *ms = 1.0f;
+    return cudaSuccess;
+}
 cudaError_t cudaDeviceSynchronize() { return cudaSuccess; }
 
 cudaError_t cudaStreamIsCapturing(cudaStream_t, cudaStreamCaptureStatus* s)
@@ -105,9 +123,19 @@ cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode)
     ++counts[4];
     return cudaSuccess;
 }
-cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t* g) { capturing = false; return make(g); }
-cudaError_t cudaGraphInstantiate(cudaGraphExec_t* e, cudaGraph_t, unsigned long long) { return make(e); }
-cudaError_t cudaGraphExecUpdate(cudaGraphExec_t, cudaGraph_t, cudaGraphExecUpdateResultInfo*) { return cudaSuccess; }
+cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t* g)
+{
+    capturing = false;
+    return make(g);
+}
+cudaError_t cudaGraphInstantiate(cudaGraphExec_t* e, cudaGraph_t, unsigned long long)
+{
+    return make(e);
+}
+cudaError_t cudaGraphExecUpdate(cudaGraphExec_t, cudaGraph_t, cudaGraphExecUpdateResultInfo*)
+{
+    return cudaSuccess;
+}
 cudaError_t cudaGraphExecDestroy(cudaGraphExec_t) { return cudaSuccess; }
 cudaError_t cudaGraphDestroy(cudaGraph_t) { return cudaSuccess; }
 cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) { ++counts[3]; return cudaSuccess; }
@@ -165,7 +193,11 @@ cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr a, int)
 }
 cudaError_t cudaGetDevice(int* d) { *d = 0; return cudaSuccess; }
 cudaError_t cudaSetDevice(int) { return cudaSuccess; }
-cudaError_t cudaDeviceGetPCIBusId(char* b, int n, int) { strncpy(b, "fake", n); return cudaSuccess; }
+cudaError_t cudaDeviceGetPCIBusId(char* b, int n, int)
+{
+    strncpy(b, "fake", n);
+    return cudaSuccess;
+}
 cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void* p)
 {
     memset(a, 0, sizeof *a);
